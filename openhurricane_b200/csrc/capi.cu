@@ -22,7 +22,7 @@
 #include "jit.h"
 #include "surrogate.cuh"
 #include "variants.h"
-#include "wcell.cuh"
+#include "wtabs.cuh"
 
 using namespace hc;
 
@@ -299,11 +299,50 @@ static bool pack_t2(const HostMech &h, const hc_mech_desc *d, T2Mech &t) {
 // the reference sums f and J in), naming slots; the third-body / fall-off
 // reactions in mechanism order.
 struct WHost {
-    std::vector<double> th, rd, eff, raw, lnu, xj;
-    std::vector<int32_t> ri, lptr, lent, tbl;
-    int nsp = 0, nrc = 0, nrc32 = 0, njob = 0, njob32 = 0;
+    std::vector<double> th, rd, eff, raw, lnu, xj, gnu;
+    std::vector<int32_t> ri, lptr, lent, tbl, rx, gslot;
+    int nsp = 0, nrc = 0, nrc32 = 0, njob = 0, njob32 = 0, gE = 0;
     double glim = 0.0;
 };
+
+// One side of a reaction as at most three unit-order factors (`none` where absent):
+// false where an order is not its stoichiometric coefficient or there are
+// more factors. `first`: multiplicity of factor 0; a repeated species' later
+// factors add no column of their own.
+static bool w_factors(const int32_t *idx, const double *nu, const double *ord, int n, int none, int trash, int *fac,
+                      int *col, int &first) {
+    int q = 0;
+    first = 1;
+    for (int k = 0; k < 3; ++k) {
+        fac[k] = none;
+        col[k] = trash;
+    }
+    for (int pass = 0; pass < 2; ++pass)      // repeated species first
+        for (int k = 0; k < n; ++k) {
+            const int c = (int)nu[k];
+            if (nu[k] != (double)c || nu[k] != ord[k] || c < 1 || c > 3) return false;
+            if ((c > 1) != (pass == 0)) continue;
+            if (c > 1 && q > 0) return false;
+            if (q + c > 3) return false;
+            if (c > 1) first = c;
+            col[q] = idx[k];
+            for (int j = 0; j < c; ++j) fac[q++] = idx[k];
+        }
+    return true;
+}
+
+// reaction r in the direct form of kernel 6 and the rate kernels: both sides as
+// unit-order factors, every species in one place only
+static bool direct_form(const HostMech &h, int r, int none, int trash, int *fac, int *col, int &mf, int &mb) {
+    const int S = HC_MAX_SIDE;
+    if (!w_factors(&h.fidx[S * r], &h.fnu[S * r], &h.ford[S * r], h.nf[r], none, trash, fac, col, mf) ||
+        !w_factors(&h.bidx[S * r], &h.bnu[S * r], &h.bord[S * r], h.nb[r], none, trash, fac + 3, col + 3, mb))
+        return false;
+    for (int a = 0; a < 6; ++a)
+        for (int b = a + 1; b < 6; ++b)
+            if (col[a] != trash && col[a] == col[b]) return false;
+    return true;
+}
 
 static bool pack_w(const HostMech &h, WHost &w) {
     if (h.nsp + 1 > 16 || h.ext) return false;
@@ -445,6 +484,43 @@ static bool pack_w(const HostMech &h, WHost &w) {
         }
     }
     w.lptr[nsp] = (int32_t)w.lnu.size();
+    // kernel 6: the direct form of each reaction and the lists in lock step
+    {
+        const int N = nsp + 1 <= 10 ? 10 : 16, trash = N + 1, P = w_parts(N);
+        w.rx.assign((size_t)2 * n32, 0);
+        for (int o = 0; o < nrc; ++o) {
+            const int r = dev[o], q = slot[o];
+            int fac[6], col[6], mf = 1, mb = 1;
+            bool ok = direct_form(h, r, kWOne, trash, fac, col, mf, mb);
+            const double sm = h.sum_stoi[r];
+            if (sm != 0.0 && sm != 1.0 && sm != -1.0) ok = false;
+            uint32_t w0 = 0, w1 = 0;
+            if (!ok) {
+                w0 = 1u << kWXgeneral;
+            } else {
+                for (int k = 0; k < 6; ++k) {
+                    w0 |= (uint32_t)fac[k] << (4 * k);
+                    w1 |= (uint32_t)col[k] << (5 * k);
+                }
+                w0 |= (h.reversible[r] ? 1u : 0u) << kWXrev;
+                w0 |= (uint32_t)((int)sm + 1) << kWXs;
+                w0 |= (uint32_t)mf << kWXmf | (uint32_t)mb << kWXmb;
+            }
+            w.rx[((size_t)(q >> 5) * 2) * 32 + (q & 31)] = (int32_t)w0;
+            w.rx[((size_t)(q >> 5) * 2 + 1) * 32 + (q & 31)] = (int32_t)w1;
+        }
+        w.gE = std::max(nsp, (nrc + P - 1) / P);
+        for (int i = 0; i < nsp; ++i) w.gE = std::max(w.gE, w.lptr[i + 1] - w.lptr[i]);
+        w.gE = (w.gE + 3) & ~3;      // read four at a time
+        w.gslot.assign((size_t)16 * w.gE, 0);
+        w.gnu.assign((size_t)16 * w.gE, 0.0);
+        for (int i = 0; i < nsp; ++i)
+            for (int e = w.lptr[i]; e < w.lptr[i + 1]; ++e) {
+                const size_t at = (size_t)16 * (e - w.lptr[i]) + i;
+                w.gslot[at] = w.lent[3 * (size_t)e] & 0xffff;
+                w.gnu[at] = w.lnu[e];
+            }
+    }
     if (w.lnu.empty()) {
         w.lent.assign(3, 0);
         w.lnu.push_back(0.0);
@@ -618,7 +694,7 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
     up(hm.xcoef.data(), 9 * (size_t)nrc, &dm.xcoef);
     up(hm.plog_ptr.data(), (size_t)nrc + 1, &dm.plog_ptr);
     {
-        // the warp-per-cell kernel's tables (nsp + 1 <= 32, the common rate forms)
+        // the warp-per-cell kernel's tables (nsp + 1 <= 16, the common rate forms)
         WHost wh;
         if (pack_w(hm, wh)) {
             WMech &w = m->w;
@@ -644,6 +720,10 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
             up(wh.lnu.data(), wh.lnu.size(), &w.lnu);
             up(wh.xj.data(), wh.xj.size(), &w.xj);
             up(wh.tbl.data(), wh.tbl.size(), &w.tbl);
+            w.gE = wh.gE;
+            up(wh.rx.data(), wh.rx.size(), &w.rx);
+            up(wh.gslot.data(), wh.gslot.size(), &w.gslot);
+            up(wh.gnu.data(), wh.gnu.size(), &w.gnu);
             up(wh.raw.data(), wh.raw.size(), &w.raw);
             m->w_ok = (rc == HC_OK);
         }
@@ -865,9 +945,9 @@ static int integrate_impl(hc_mech_t m, const hc_opts *opts, int64_t ncells, doub
     // automatic choice (kernel 0): the warp-per-cell kernel wherever it takes
     // the mechanism (the fastest on the batched workload: 1.14e8 Newton
     // iterations/s against 0.6e8 for the cell group), else the cell group
-    const bool auto_w = m->kernel == 0 && m->w_ok && opts->reactor == 0;
+    const bool auto_w = m->kernel == 0 && m->w_ok && launch_w_fits(m->w, P);
     if (m->kernel == 6 || auto_w) {
-        if (!m->w_ok || opts->reactor != 0)
+        if (!auto_w && (!m->w_ok || opts->reactor != 0))
             return fail(HC_E_UNSUPPORTED,
                         "warp-per-cell kernel needs nsp + 1 <= 16, the constant-pressure reactor and no "
                         "SRI, explicit reverse (REV), PLOG, HIGH, LT, JAN, FIT1 or collision rate laws");

@@ -4,12 +4,15 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <string>
 
 #include "../../include/hurchem_b200.h"
 #include "integrator.cuh"
 
 namespace hc {
+
+constexpr size_t kMaxSmem = 227 * 1024;   // shared memory a block can have
 
 #define HC_LCUDA(call)                                                  \
     do {                                                                \
@@ -19,6 +22,21 @@ namespace hc {
             return HC_E_CUDA;                                           \
         }                                                               \
     } while (0)
+
+// lets a kernel's blocks have up to kMaxSmem of shared memory, once per device
+// (the attribute stays; the call costs a launch's worth of host time)
+template <auto Kernel>
+int allow_smem(std::string &err) {
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    HC_LCUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(done.load(std::memory_order_acquire) & bit)) {
+        HC_LCUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+        done.fetch_or(bit, std::memory_order_release);
+    }
+    return HC_OK;
+}
 
 template <int N, int G>
 struct Launch {

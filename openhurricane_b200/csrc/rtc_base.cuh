@@ -57,20 +57,18 @@ __device__ __forceinline__ double pow_n(double x, double y) {
     return pow_out(x, y);
 }
 
-// 1/b without a branch to a slow path: the hardware approximation (PTX
-// rcp.approx.ftz.f64) refined by three Newton-Raphson steps r <- r + r (1 - b r),
-// each of which doubles the number of correct bits (Markstein, IBM J. Res.
-// Dev. 34 (1990) 111-119); the result is within a few ulp of the correctly
-// rounded reciprocal. Zero, infinity and NaN keep the approximation's own
-// result (+-inf, +-0, NaN), as do subnormal b (flushed: +-inf).
+// 1/b without a branch to a slow path: the hardware approximation r (PTX
+// rcp.approx.ftz.f64, 2^-20) and one cubic step r (1 + e + e^2), e = 1 - b r,
+// which triples its correct bits in three dependent operations; the result is
+// within an ulp of the correctly rounded reciprocal. Zero, infinity and NaN
+// keep the approximation's own result (+-inf, +-0, NaN), as do subnormal b
+// (flushed: +-inf).
 __device__ __forceinline__ double frcp(double b) {
 #ifdef __CUDA_ARCH__
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    double x = r;
-    x = fma(x, fma(-b, x, 1.0), x);
-    x = fma(x, fma(-b, x, 1.0), x);
-    x = fma(x, fma(-b, x, 1.0), x);
+    const double e = fma(-b, r, 1.0);
+    const double x = fma(r, fma(e, e, e), r);
     return (r != 0.0 && !isinf(r)) ? x : r;
 #else
     return 1.0 / b;   // host builds of the device code (arithmetic checks on the CPU)
@@ -361,7 +359,7 @@ struct IntegratorParams {
     double atol_inc, rtol_inc, T_threshold, T_alpha, T_beta, dt_max;
     double err_accept_limit;     // pow(maxscale/safescale, -1/alphainc)
     int64_t max_newton_total;
-    int32_t reactor;             // 0 constant pressure, 1 constant volume (cell group only)
+    int32_t reactor;             // 0 constant pressure, 1 constant volume (cell group, warp and block per cell)
 };
 
 struct CellIO {

@@ -35,7 +35,7 @@
 #pragma once
 
 #include "t1_body.cuh"
-#include "wcell.cuh"
+#include "wtabs.cuh"
 
 namespace hc {
 

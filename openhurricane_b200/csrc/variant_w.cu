@@ -10,25 +10,54 @@
 
 namespace hc {
 
+// most warps per block whose shared memory fits (0: not even one)
 template <int N>
+static int w_warps(const WMech &m, const IntegratorParams &P) {
+    int w = kWWarps;
+    while (w > 0 && w6_smem_bytes<N>(m, w, P.auto_update_jacobian != 0) > kMaxSmem) w /= 2;
+    return w;
+}
+
+bool launch_w_fits(const WMech &m, const IntegratorParams &P) {
+    return (m.nsp + 1 <= 10 ? w_warps<10>(m, P) : w_warps<16>(m, P)) > 0;
+}
+
+template <int N, int BLOCKS>
 static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
                     cudaStream_t st, std::string &err) {
-    auto kern = integrate_w_kernel<N>;
-    const size_t sm = w_tables_bytes(m.nsp, m.nrc, m.nrc32, m.nent, m.ntb, m.njob32) +
-                      WSmem<N>::bytes(m.nrc32, m.njob32) * kWWarps;
-    HC_LCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    auto kern = integrate_w_kernel<N, BLOCKS>;
+    const int warps = w_warps<N>(m, P);
+    const size_t sm = w6_smem_bytes<N>(m, warps, P.auto_update_jacobian != 0);
     int per_sm = 0;
-    HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWWarps, sm));
+    if (warps > 0) {
+        if (int rc = allow_smem<integrate_w_kernel<N, BLOCKS>>(err)) return rc;
+        HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, sm));
+    }
     if (per_sm < 1) {
         err = "warp-per-cell kernel does not fit on an SM";
         return HC_E_UNSUPPORTED;
     }
-    const int64_t blocks_needed = (io.nqueue + kWWarps - 1) / kWWarps;
-    const int64_t grid = std::min<int64_t>(blocks_needed, (int64_t)per_sm * num_sms);
+    // fewer cells than warps: one block per cell until every SM has its blocks,
+    // so that few cells do not share an SM's issue slots
+    const int64_t grid = std::min<int64_t>(io.nqueue, (int64_t)per_sm * num_sms);
     if (grid <= 0) return HC_OK;
-    kern<<<(unsigned)grid, 32 * kWWarps, sm, st>>>(m, P, io);
+    kern<<<(unsigned)grid, 32 * warps, sm, st>>>(m, P, io);
     HC_LCUDA(cudaGetLastError());
     return HC_OK;
+}
+
+// One block of eight warps per SM and no spills, or two with 128 registers a thread.
+// A flow step ends with its stiffest cells, whose iterations the first build does in
+// 4.8 us against 6.5 us; only when the cells go round many times does the second's
+// larger number in flight pay. Dirichlet cells at 1e-7 s and mixed cells at 1e-6 s, ms,
+// first / second build: 12,288 cells 118 / 162 and 79 / 97; 18,944: 182 / 182 and
+// 118 / 108; 37,888: 361 / 318 and 239 / 234; 131,072 mixed: 779 / 674. So the line lies
+// at 8 cells for each of the second's warps.
+template <int N>
+static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
+                    cudaStream_t st, std::string &err) {
+    if (io.nqueue < (int64_t)8 * 2 * kWWarps * num_sms) return launch_w<N, 1>(m, num_sms, P, io, st, err);
+    return launch_w<N, 2>(m, num_sms, P, io, st, err);
 }
 
 int launch_integrate_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
