@@ -20,6 +20,7 @@
 #include "../../include/hurchem_b200.h"
 #include "integrator_t2.cuh"
 #include "jit.h"
+#include "rates.cuh"
 #include "surrogate.cuh"
 #include "variants.h"
 #include "wtabs.cuh"
@@ -103,6 +104,9 @@ struct hc_mech_s {
     // the warp-per-cell kernel's tables (kernel 6)
     WMech w{};
     bool w_ok = false;
+    // the rate kernels' tables
+    RMech r{};
+    bool r_ok = false;
 };
 
 namespace {
@@ -341,6 +345,87 @@ static bool direct_form(const HostMech &h, int r, int none, int trash, int *fac,
     for (int a = 0; a < 6; ++a)
         for (int b = a + 1; b < 6; ++b)
             if (col[a] != trash && col[a] == col[b]) return false;
+    return true;
+}
+
+// The mechanism in the rate kernels' tables (rates.cuh), if every reaction has
+// the direct form. A third body's concentration is the sum over all species
+// plus the entries' differences from 1, or the entries alone: the shorter
+// list, but the sum only where no efficiency is below 1/4, so that a species
+// that counts little is not the small difference of large numbers.
+struct RHost {
+    std::vector<int4> code;
+    std::vector<double4> rate;
+    std::vector<double> th, eval, fall;
+    std::vector<int32_t> eidx;
+};
+
+static bool pack_r(const HostMech &h, RHost &o) {
+    if (h.ext || h.nsp > 63) return false;
+    const int nsp = h.nsp, nrc = h.nrc, none = nsp, trash = 255;
+    for (int i = 0; i < nsp; ++i) {
+        for (int k = 0; k < 3; ++k) o.th.push_back(h.Trange[3 * i + k]);
+        o.th.push_back(h.W[i]);
+        o.th.push_back(1.0 / h.W[i]);
+        for (int rg = 0; rg < 2; ++rg) {
+            const double *a = &h.nasa[14 * i + 7 * rg];
+            const double div[5] = {1.0, 2.0, 6.0, 12.0, 20.0};
+            for (int k = 0; k < 6; ++k) o.th.push_back(a[k] * h.W[i] / kRu);
+            for (int k = 0; k < 5; ++k) o.th.push_back(a[k] / div[k]);
+            o.th.push_back(a[5]);
+            o.th.push_back(a[6]);
+        }
+    }
+    for (int r = 0; r < nrc; ++r) {
+        int fac[6], col[6], mf = 1, mb = 1;
+        if (!direct_form(h, r, none, trash, fac, col, mf, mb)) return false;
+        const int type = h.rate_type[r];
+        int4 c;
+        c.x = fac[0] | fac[1] << 8 | fac[2] << 16 | type << 24;
+        c.y = fac[3] | fac[4] << 8 | fac[5] << 16;
+        int last = 7;
+        unsigned z = 0;
+        for (int k = 0; k < 6; ++k) {
+            if (col[k] != trash) z |= 1u << k;
+            if (col[k] == nsp - 1) last = k;
+        }
+        z |= (unsigned)mf << kRmf | (unsigned)mb << kRmb | (h.reversible[r] ? 1u : 0u) << kRrev;
+        z |= (unsigned)last << kRlast;
+        const size_t e0 = o.eidx.size(), f0 = o.fall.size() / kRFall;
+        if (type != HC_RATE_ARRHENIUS) {
+            const double *e = &h.eff[(size_t)r * nsp];
+            int n0 = 0, n1 = 0;
+            double low = 1.0;
+            for (int i = 0; i < nsp; ++i) {
+                n0 += e[i] != 0.0;
+                n1 += e[i] != 1.0;
+                low = std::min(low, e[i]);
+            }
+            const bool all = low >= 0.25 && n1 < n0;
+            for (int i = 0; i < nsp; ++i) {
+                if (e[i] == (all ? 1.0 : 0.0)) continue;
+                o.eidx.push_back(i);
+                o.eval.push_back(all ? e[i] - 1.0 : e[i]);
+            }
+            z |= (all ? 1u : 0u) << kRall | (unsigned)(o.eidx.size() - e0) << kRneff;
+        }
+        if (type >= HC_RATE_LINDEMANN) {
+            const bool troe = type != HC_RATE_LINDEMANN;
+            const double *t = &h.troe[4 * (size_t)r];
+            for (int k = 0; k < 3; ++k) o.fall.push_back(h.arr0[3 * (size_t)r + k]);
+            o.fall.push_back(troe ? t[0] : 0.0);
+            o.fall.push_back(troe ? 1.0 / t[1] : 0.0);
+            o.fall.push_back(troe ? 1.0 / t[2] : 0.0);
+            o.fall.push_back(troe ? t[3] : 0.0);
+            o.fall.push_back(0.0);
+        }
+        if (e0 >= (1u << 16) || f0 >= (1u << 15)) return false;
+        c.z = (int)z;
+        c.w = (int)((unsigned)e0 | (unsigned)f0 << 16);
+        o.code.push_back(c);
+        o.rate.push_back(make_double4(h.arr[3 * (size_t)r], h.arr[3 * (size_t)r + 1], h.arr[3 * (size_t)r + 2],
+                                      h.sum_stoi[r]));
+    }
     return true;
 }
 
@@ -726,6 +811,21 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
             up(wh.gnu.data(), wh.gnu.size(), &w.gnu);
             up(wh.raw.data(), wh.raw.size(), &w.raw);
             m->w_ok = (rc == HC_OK);
+        }
+    }
+    {
+        RHost rh;
+        if (pack_r(hm, rh)) {
+            RMech &r = m->r;
+            r.nsp = hm.nsp;
+            r.nrc = hm.nrc;
+            up(rh.code.data(), rh.code.size(), &r.code);
+            up(rh.rate.data(), rh.rate.size(), &r.rate);
+            up(rh.th.data(), rh.th.size(), &r.th);
+            up(rh.eidx.data(), rh.eidx.size(), &r.eidx);
+            up(rh.eval.data(), rh.eval.size(), &r.eval);
+            up(rh.fall.data(), rh.fall.size(), &r.fall);
+            m->r_ok = (rc == HC_OK);
         }
     }
     up(hm.plog_p.data(), hm.plog_p.size(), &dm.plog_p);
@@ -1150,6 +1250,8 @@ int hc_source_terms(hc_mech_t m, int64_t n, const double *T, const double *p, co
     if (n <= 0) return HC_OK;
     if (!T || !p || !rho || !Y || !Ri) return fail(HC_E_INVALID, "null field");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (m->r_ok && rates_fit(m->r.nsp, m->r.nrc, false))
+        return launch_rates(m->r, m->dm, m->num_sms, n, T, rho, Y, Ri, nullptr, st, g_err);
     HC_DISPATCH(m, source, m->dm, n, T, p, rho, Y, Ri, st, g_err);
 }
 
@@ -1161,6 +1263,8 @@ int hc_source_terms_imp(hc_mech_t m, int64_t n, const double *T, const double *p
     if (!T || !p || !rho || !Y || !Ri || !diag) return fail(HC_E_INVALID, "null field");
     if (m->dm.nsp < 2) return fail(HC_E_INVALID, "point-implicit terms need at least 2 species");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (m->r_ok && rates_fit(m->r.nsp, m->r.nrc, true))
+        return launch_rates(m->r, m->dm, m->num_sms, n, T, rho, Y, Ri, diag, st, g_err);
     HC_DISPATCH(m, srcimp, m->dm, n, T, p, rho, Y, Ri, diag, st, g_err);
 }
 
