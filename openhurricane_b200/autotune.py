@@ -7,7 +7,9 @@ kernel 1 = thread per cell (nsp + 1 <= 16; block 32/64/128 threads),
 kernel 3 = thread per cell generated for the mechanism (same limits),
 kernel 4 = compact thread per cell (mechanism in the constant bank),
 kernel 2 = cell group (32 lanes per cell up to 32 unknowns, 64 above; the
-block argument is ignored).
+block argument is ignored), and the automatic choice (kernel 0) for more than
+16 unknowns and for the constant-volume reactor, which only it runs on the
+block per cell and the warp per cell.
 Each candidate integrates the same sample of cells (a strided subset of the
 caller's cells, restored before every trial) once untimed and `repeats`
 times timed with CUDA events on the current stream; the fastest median wins
@@ -81,7 +83,9 @@ def autotune(mech, T: torch.Tensor, p: torch.Tensor, rho: torch.Tensor, Y: torch
         _capi.check(rc, "hc_integrate")
 
     results = []
-    for kernel, block in (cands or candidates(mech.nsp)):
+    # the automatic choice has a kernel of its own where kernels 1 and 3 to 7 do not apply
+    auto = [(0, 64)] if mech.nsp + 1 > 16 or o.reactor != 0 else []
+    for kernel, block in (cands or auto + candidates(mech.nsp)):
         try:
             mech.set_tuning(kernel, block)
             run()

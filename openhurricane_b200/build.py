@@ -22,7 +22,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"]
 # translation units: the C ABI plus one file per kernel variant
 UNITS = ["capi.cu", "variant_10.cu", "variant_16.cu", "variant_32.cu", "variant_54.cu",
          "variant_64.cu", "variant_t1.cu", "variant_t2.cu", "props.cu", "probe.cu", "mlp.cu", "surrogate.cu", "jit.cu",
-         "aos.cu", "jit_t3.cu", "variant_w.cu", "rates.cu"]
+         "aos.cu", "jit_t3.cu", "variant_w.cu", "variant_b.cu", "rates.cu"]
 # headers handed to NVRTC with the generated kernels (embedded as strings)
 JIT_HEADERS = ["rtc_base.cuh", "t1_body.cuh", "t3_base.cuh", "t4_cell.cuh"]
 

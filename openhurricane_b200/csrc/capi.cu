@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "../../include/hurchem_b200.h"
+#include "bcell.cuh"
 #include "integrator_t2.cuh"
 #include "jit.h"
 #include "rates.cuh"
@@ -107,6 +108,9 @@ struct hc_mech_s {
     // the rate kernels' tables
     RMech r{};
     bool r_ok = false;
+    // the block-per-cell kernels' tables
+    BMech b{};
+    bool b_ok = false;
 };
 
 namespace {
@@ -426,6 +430,126 @@ static bool pack_r(const HostMech &h, RHost &o) {
         o.rate.push_back(make_double4(h.arr[3 * (size_t)r], h.arr[3 * (size_t)r + 1], h.arr[3 * (size_t)r + 2],
                                       h.sum_stoi[r]));
     }
+    return true;
+}
+
+// The block-per-cell kernels' tables (bcell.cuh) from the rate kernels': which
+// lanes evaluate which reactions, and every nonzero of J, f and the column of T
+// (and each row's third-body sum) as a list of signed terms.
+struct BHost {
+    BMech b{};
+    std::vector<int32_t> task, tptr, gptr, pair;
+    std::vector<uint32_t> dst;
+    std::vector<uint2> term;
+};
+
+// the items to the least loaded of the warps, longest first
+static std::vector<std::vector<int>> balance(const std::vector<double> &cost) {
+    std::vector<int> by(cost.size());
+    for (size_t i = 0; i < by.size(); ++i) by[i] = (int)i;
+    std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    std::vector<std::vector<int>> out(kBWarps);
+    std::vector<double> load(kBWarps, 0.0);
+    for (int i : by) {
+        const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        out[w].push_back(i);
+        load[w] += cost[i];
+    }
+    return out;
+}
+
+static bool pack_b(const RHost &r, int nsp, BHost &o) {
+    const int nrc = (int)r.code.size(), N = nsp + 1;
+    int F = 2, R = 2;
+    for (const int4 &c : r.code) {
+        if (((c.x >> 16) & 255) != nsp) F = 3;
+        if (((c.y >> 16) & 255) != nsp) R = 3;
+    }
+    BMech &b = o.b;
+    b.nf = F;
+    b.stride = kBd + F + R;
+    b.ndv = (int)r.eidx.size();
+    b.ld = (nsp + 2) | 1;
+    const int zero = b.zero = std::max(nrc * b.stride + b.ndv, b_ucol(N));
+    if (N > 64 || zero >= (1 << 15)) return false;
+    // reactions, the costly rate forms first, in tasks of 32
+    std::vector<int> order(nrc);
+    for (int i = 0; i < nrc; ++i) order[i] = i;
+    auto type = [&](int i) { return r.code[i].x >> 24; };
+    auto cls = [&](int i) { return type(i) >= HC_RATE_LINDEMANN ? 0 : type(i) == HC_RATE_THIRD_BODY ? 1 : 2; };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cls(x) < cls(y); });
+    std::vector<double> cost;
+    for (int i = 0; i < nrc; i += 32) cost.push_back(cls(order[i]) == 0 ? 5.0 : cls(order[i]) == 1 ? 1.5 : 1.0);
+    o.tptr.assign(1, 0);
+    for (const auto &list : balance(cost)) {
+        for (int t : list)
+            for (int k = 0; k < 32; ++k) o.task.push_back(32 * t + k < nrc ? order[32 * t + k] : -1);
+        o.tptr.push_back((int)o.task.size() / 32);
+    }
+    // terms: place in the records, sign
+    std::vector<std::vector<uint32_t>> item(nsp * b.ld + nsp);   // J region, then the rows' sums
+    for (int q = 0; q < nrc; ++q) {
+        const int4 c = r.code[q];
+        int sp[6], nu[6], at[6];
+        for (int k = 0; k < 6; ++k) {
+            const int word = k < 3 ? c.x : c.y;
+            sp[k] = ((c.z >> k) & 1) ? (word >> (8 * (k % 3))) & 255 : -1;
+            nu[k] = k == 0 ? -((c.z >> kRmf) & 3) : k == 3 ? (c.z >> kRmb) & 3 : k < 3 ? -1 : 1;
+            at[k] = q * b.stride + kBd + (k < 3 ? k : F + k - 3);
+        }
+        auto add = [&](int to, int n, int place) {
+            for (int k = 0; k < std::abs(n); ++k) item[to].push_back((uint32_t)place | (n < 0 ? 0x8000u : 0u));
+        };
+        for (int k = 0; k < 6; ++k) {
+            if (sp[k] < 0) continue;
+            const int i = sp[k];
+            add(i * b.ld + N, nu[k], q * b.stride + kBq);
+            add(i * b.ld + nsp, nu[k], q * b.stride + kBdq);
+            for (int j = 0; j < 6; ++j)
+                if (sp[j] >= 0) add(i * b.ld + sp[j], nu[k], at[j]);
+            if (type(q) == HC_RATE_ARRHENIUS) continue;
+            if ((c.z >> kRall) & 1) add(nsp * b.ld + i, nu[k], q * b.stride + kBg);
+            const int e0 = c.w & 0xffff, ne = (c.z >> kRneff) & 255;
+            for (int e = e0; e < e0 + ne; ++e) add(i * b.ld + r.eidx[e], nu[k], nrc * b.stride + e);
+        }
+    }
+    std::vector<int> ids;
+    for (size_t i = 0; i < item.size(); ++i)
+        if (!item[i].empty()) ids.push_back((int)i);
+    std::stable_sort(ids.begin(), ids.end(), [&](int x, int y) { return item[x].size() > item[y].size(); });
+    // 64 items a pair of groups: lane l has items l and 32 + l, as long as the longest
+    cost.clear();
+    for (size_t i = 0; i < ids.size(); i += 64) cost.push_back(2.0 + (item[ids[i]].size() + 1) / 2);
+    const uint32_t nothing = (uint32_t)zero | (uint32_t)zero << 16;
+    if (nsp * b.ld >= (int)kBRow) return false;
+    o.gptr.assign(1, 0);
+    for (const auto &list : balance(cost)) {
+        for (int g : list) {
+            const int words = ((int)item[ids[64 * (size_t)g]].size() + 1) / 2, base = (int)o.term.size() / 32;
+            if (base >= (1 << 16) || words >= (1 << 15)) return false;
+            o.term.resize(o.term.size() + 32 * (size_t)words, make_uint2(nothing, nothing));
+            for (int l = 0; l < 32; ++l) {
+                uint32_t to[2];
+                for (int half = 0; half < 2; ++half) {
+                    const size_t at = 64 * (size_t)g + 32 * half + l;
+                    to[half] = (uint32_t)(nsp * b.ld);          // a place nothing reads
+                    if (at >= ids.size()) continue;
+                    const int id = ids[at];
+                    to[half] = id < nsp * b.ld ? (uint32_t)id : kBRow | (uint32_t)(id - nsp * b.ld);
+                    for (size_t k = 0; k < item[id].size(); ++k) {
+                        uint2 &v = o.term[32 * (size_t)(base + (int)k / 2) + l];
+                        uint32_t &w = half ? v.y : v.x;
+                        w = (k & 1) ? (w & 0xffffu) | item[id][k] << 16 : (w & 0xffff0000u) | item[id][k];
+                    }
+                }
+                o.dst.push_back(to[0] | to[1] << 16);
+            }
+            o.pair.push_back(base | words << 16);
+        }
+        o.gptr.push_back((int)o.pair.size());
+    }
+    b.npair = (int)o.pair.size();
+    b.nword = (int)o.term.size() / 32;
     return true;
 }
 
@@ -826,6 +950,18 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
             up(rh.eval.data(), rh.eval.size(), &r.eval);
             up(rh.fall.data(), rh.fall.size(), &r.fall);
             m->r_ok = (rc == HC_OK);
+            BHost bh;
+            if (pack_b(rh, hm.nsp, bh)) {
+                BMech &b = m->b;
+                b = bh.b;
+                up(bh.task.data(), bh.task.size(), &b.task);
+                up(bh.tptr.data(), bh.tptr.size(), &b.tptr);
+                up(bh.gptr.data(), bh.gptr.size(), &b.gptr);
+                up(bh.pair.data(), bh.pair.size(), &b.pair);
+                up(bh.dst.data(), bh.dst.size(), &b.dst);
+                up(bh.term.data(), bh.term.size(), &b.term);
+                m->b_ok = (rc == HC_OK) && launch_b_fits(m->r, b);
+            }
         }
     }
     up(hm.plog_p.data(), hm.plog_p.size(), &dm.plog_p);
@@ -1053,6 +1189,9 @@ static int integrate_impl(hc_mech_t m, const hc_opts *opts, int64_t ncells, doub
                         "SRI, explicit reverse (REV), PLOG, HIGH, LT, JAN, FIT1 or collision rate laws");
         return launch_integrate_w(m->w, m->num_sms, P, io, st, g_err);
     }
+    // larger mechanisms: the block-per-cell kernel where it takes the reactions
+    if (m->kernel == 0 && N > 16 && m->b_ok && !opts->auto_update_jacobian)
+        return launch_integrate_b(m->r, m->b, m->num_sms, P, io, st, g_err);
     if (m->kernel == 5 && !t1_ok)
         return fail(HC_E_UNSUPPORTED,
                     "direct-assembly thread-per-cell kernel needs nsp <= 15, autoUpdateJacobian off, "
@@ -1241,6 +1380,8 @@ int hc_rhs_jacobian(hc_mech_t m, int64_t n, const double *c, const double *T, co
     if (n <= 0) return HC_OK;
     if (!c || !T || !p) return fail(HC_E_INVALID, "null field");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (m->b_ok && m->dm.nsp + 1 > 16)
+        return launch_jacobian_b(m->r, m->b, m->num_sms, n, c, T, dydt, J, st, g_err);
     HC_DISPATCH(m, rhsjac, m->dm, n, c, T, p, dydt, J, st, g_err);
 }
 

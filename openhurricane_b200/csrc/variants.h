@@ -39,6 +39,14 @@ struct WMech;
 // the warp-per-cell integrator (variant_w.cu, wcell.cuh)
 int launch_integrate_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
                        cudaStream_t st, std::string &err);
+// the block-per-cell integrator and Jacobian (variant_b.cu, bcell.cuh)
+struct RMech;
+struct BMech;
+bool launch_b_fits(const RMech &m, const BMech &b);
+int launch_integrate_b(const RMech &m, const BMech &b, int num_sms, const IntegratorParams &P, const CellIO &io,
+                       cudaStream_t st, std::string &err);
+int launch_jacobian_b(const RMech &m, const BMech &b, int num_sms, int64_t n, const double *c, const double *T,
+                      double *dydt, double *J, cudaStream_t st, std::string &err);
 // whether its shared memory holds the mechanism
 bool launch_w_fits(const WMech &m, const IntegratorParams &P);
 int launch_integrate_s(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
