@@ -983,28 +983,32 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
     if (d->eps_k) up(d->eps_k, nsp, &dm.eps_k);
     if (d->sigma) up(d->sigma, nsp, &dm.sigma);
     if (d->eps_k && d->sigma) {
-        // pair constants of kineticTheory::Di (kineticTheory.cpp:126-141) and of
-        // the Wilke factors (transportList.cpp:31-56), with the host libm
-        const size_t nn = (size_t)nsp * nsp;
-        std::vector<double> pD(nn), pP(nn), pR(nn), pPhi(nn), pW(nn);
-        const double c8 = 1.0 / std::sqrt(8.0);
+        // constants of kineticTheory::Di (kineticTheory.cpp:126-141) and of the
+        // Wilke factors (transportList.cpp:31-56), with the host libm, in the
+        // property kernel's layout (DevMech::ptab)
+        const int NB = (nsp + 3) / 4;
+        const size_t tab = (size_t)4 * NB * nsp;
+        std::vector<double> t(3 * tab + 4 * (size_t)NB + 6 * (size_t)nsp, 0.0);
         for (int i = 0; i < nsp; ++i) {
-            const double invW = 1.0 / d->W[i];
             for (int j = 0; j < nsp; ++j) {
-                const size_t k = (size_t)i * nsp + j;
+                const size_t k = ((size_t)(i / 4) * nsp + j) * 4 + i % 4;
                 const double sij = 0.5 * (d->sigma[i] + d->sigma[j]);
-                pD[k] = 1.858e-7 * std::sqrt(invW + 1.0 / d->W[j]) / (sij * sij) * 1.01325e5;
-                pR[k] = 1.0 / std::sqrt(d->eps_k[i] * d->eps_k[j]);
-                pP[k] = std::exp(-0.145 * std::log(pR[k]));
-                pPhi[k] = c8 / std::sqrt(1.0 + d->W[i] / d->W[j]);
-                pW[k] = std::sqrt(d->W[i] / d->W[j]);
+                const double pD = 1.858e-7 * std::sqrt(1.0 / d->W[i] + 1.0 / d->W[j]) / (sij * sij) * 1.01325e5;
+                t[k] = 1.0 / std::sqrt(8.0 * (1.0 + d->W[i] / d->W[j]));
+                if (j == i) continue;
+                t[tab + k] = 1.0 / pD;
+                t[2 * tab + k] = std::exp(0.145 * 0.5 * std::log(d->eps_k[i] * d->eps_k[j]));
             }
+            t[3 * tab + i] = 1.0 / std::sqrt(d->eps_k[i]);
+            double *q = &t[3 * tab + 4 * (size_t)NB + 6 * (size_t)i];
+            q[0] = 1.0 / d->eps_k[i];
+            q[1] = std::exp(0.145 * std::log(d->eps_k[i]));
+            q[2] = std::sqrt(d->W[i]) / (d->sigma[i] * d->sigma[i]);
+            q[3] = std::sqrt(std::sqrt(d->W[i]));
+            q[4] = 1.0 / d->W[i];
+            q[5] = kRu / d->W[i];
         }
-        up(pD.data(), nn, &dm.pair_D);
-        up(pP.data(), nn, &dm.pair_Dpow);
-        up(pR.data(), nn, &dm.pair_r);
-        up(pPhi.data(), nn, &dm.pair_phi);
-        up(pW.data(), nn, &dm.pair_w);
+        up(t.data(), t.size(), &dm.ptab);
     }
     if (rc == HC_OK) {
         void *q = nullptr;

@@ -39,12 +39,11 @@ struct DevMech {
     // kinetic-theory transport
     const int32_t *geom;
     const double *eps_k, *sigma;
-    // pair constants of the mixture-averaged transport, [nsp*nsp] (i*nsp + j)
-    const double *pair_D;     // 1.858e-7 sqrt(1/Wi + 1/Wj) / sigma_ij^2 * Patm
-    const double *pair_Dpow;  // (1/sqrt(eps_i eps_j))^-0.145
-    const double *pair_r;     // 1/sqrt(eps_i eps_j)
-    const double *pair_phi;   // (1/sqrt 8) / sqrt(1 + Wi/Wj)
-    const double *pair_w;     // sqrt(Wi/Wj)
+    // the property kernel's tables, [row block of 4][j][4 rows] each: 1/sqrt(8 (1 + Wi/Wj)),
+    // 1/(1.858e-7 sqrt(1/Wi + 1/Wj) / sigma_ij^2 * Patm) and (1/sqrt(eps_i eps_j))^-0.145,
+    // the last two zero for j = i; then 1/sqrt(eps)
+    // of each row and per species 1/eps, (1/eps)^-0.145, sqrt(W)/sigma^2, W^(1/4), 1/W, Ru/W
+    const double *ptab;
 };
 
 template <typename V>
@@ -102,7 +101,7 @@ __device__ __forceinline__ void species_cp_h(const DevMech &m, int i, double T, 
     const bool out = (T < tl || T > th);
     const double T0 = out ? hmin(hmax(T, tl), th) : T;
     cp = ((((a4 * T0 + a3) * T0 + a2) * T0 + a1) * T0 + a0);
-    h = ((((a4 / 5.0 * T0 + a3 / 4.0) * T0 + a2 / 3.0) * T0 + a1 / 2.0) * T0 + a0) * T0 + a5;
+    h = ((((a4 * 0.2 * T0 + a3 * 0.25) * T0 + a2 * (1.0 / 3.0)) * T0 + a1 * 0.5) * T0 + a0) * T0 + a5;
     if (out) h += cp * (T - T0);
 }
 
