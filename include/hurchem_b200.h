@@ -180,8 +180,10 @@ void hc_default_opts(hc_opts *opts);
 
 /*
  * Kernel selection for hc_integrate*: kernel 0 = automatic (the warp per
- * cell, kernel 6, wherever it takes the mechanism and the reactor, else the
- * cell group: their lanes share each Newton iteration of one cell, which
+ * cell, kernel 6, wherever it takes the mechanism, for either reactor; above
+ * 16 unknowns a block per cell where the reactions have its form and
+ * autoUpdateJacobian is off; else the cell group: they share each Newton
+ * iteration of one cell among threads, which
  * bounds the step's duration when per-cell costs are uneven), 1 = table-driven thread per
  * cell, 2 = cell group (32 lanes up to 32 unknowns, 64 above),
  * 3 = thread per cell generated for this mechanism (every index and
@@ -192,7 +194,7 @@ void hc_default_opts(hc_opts *opts);
  * I - dt J assembled column by column from register-held rates and written
  * once per entry, no divisions on the common path and a small instruction
  * footprint (NVRTC on first use, like 3), 6 = warp per cell (one cell per
- * warp, lane i holding element i and row i of the Newton matrix; nsp + 1 <= 16),
+ * warp, each row of the Newton matrix over several lanes; nsp + 1 <= 16),
  * 7 = segment per cell (32 / (nsp + 1) cells per warp, one per segment of
  * nsp + 1 lanes, each segment with its own step-control state; nsp + 1 <= 16);
  * block = threads per block of the thread-per-cell kernels (32, 64 or 128;
@@ -201,8 +203,8 @@ void hc_default_opts(hc_opts *opts);
  * The thread-per-cell kernels (1, 3, 4, 5) take nsp <= 15, the constant-pressure
  * reactor and the common rate forms (Arrhenius, third body, Lindemann / Troe
  * fall-off); a call that asks for one of them outside that range fails with
- * HC_E_UNSUPPORTED; kernels 6 and 7 take the same rate forms and reactor,
- * and autoUpdateJacobian. The cell group takes everything hc_mech_create accepts.
+ * HC_E_UNSUPPORTED; kernels 6 and 7, asked for by number, take the same rate
+ * forms and reactor, and autoUpdateJacobian. The cell group takes everything hc_mech_create accepts.
  * No reference counterpart.
  */
 int hc_set_tuning(hc_mech_t mech, int kernel, int block);
@@ -548,6 +550,11 @@ int hc_gemm_bf16_tn(const void *A, const void *B, int M, int N, int K, const flo
  * ln max(Y_1, 1e-20) .. ln max(Y_nsp, 1e-20), ln(dt*dt_factor)):
  * (value - mean[j]) * inv_std[j].
  *
+ * hc_surrogate_ensemble: mean[n][n_out] of the predictions preds[n_nets][n][n_out]
+ * and per cell the ensemble's disagreement, the largest over the outputs of
+ * (max - min) * out_std[j] / (j == 0 ? spread_T : spread_Y); NaN where a
+ * prediction is NaN.
+ *
  * hc_surrogate_gate: pred[n][nsp+1] is the network's normalised increment
  * (dT, dY_1..dY_nsp) over the flow step (de-normalised with out_mean /
  * out_std). Per cell, in FP64: dY is projected onto the element-conserving
@@ -574,6 +581,9 @@ typedef struct hc_gate_opts {
 int hc_surrogate_features(hc_mech_t mech, int64_t n, const double *T, const double *p,
                           const double *Y, const double *dt, double dt_factor, const double *mean,
                           const double *inv_std, float *X, void *stream);
+int hc_surrogate_ensemble(int64_t n, int n_out, int n_nets, const float *preds,
+                          const double *out_std, double spread_T, double spread_Y, float *mean,
+                          float *spread, void *stream);
 int hc_surrogate_gate(hc_mech_t mech, int64_t n, double *T, const double *p, double *rho,
                       double *Y, const float *pred, const float *X, const double *out_mean,
                       const double *out_std, const double *proj, const double *elem, int nel,

@@ -159,6 +159,8 @@ SIGNATURES = {
     "hc_mlp_forward": (C.c_int, [_VP, _VP, C.c_int64, _VP, _VP]),
     "hc_mlp_check": (C.c_int, [_VP, _VP]),
     "hc_surrogate_features": (C.c_int, [_VP, C.c_int64] + [_VP] * 4 + [C.c_double] + [_VP] * 4),
+    "hc_surrogate_ensemble": (C.c_int, [C.c_int64, C.c_int, C.c_int, _VP, _VP, C.c_double, C.c_double, _VP, _VP,
+                                        _VP]),
     "hc_surrogate_gate": (C.c_int, [_VP, C.c_int64] + [_VP] * 10 + [C.c_int] + [_VP] * 6),
     "hc_gemm_bf16_tn": (C.c_int, [_VP, _VP, C.c_int, C.c_int, C.c_int, _VP, C.c_int, _VP, _VP]),
 }

@@ -1508,6 +1508,14 @@ int hc_surrogate_features(hc_mech_t m, int64_t n, const double *T, const double 
                            static_cast<cudaStream_t>(stream));
 }
 
+int hc_surrogate_ensemble(int64_t n, int n_out, int n_nets, const float *preds, const double *out_std,
+                          double spread_T, double spread_Y, float *mean, float *spread, void *stream) {
+    if (n <= 0) return HC_OK;
+    if (!preds || !out_std || !mean || !spread) return fail(HC_E_INVALID, "null field");
+    if (n_out <= 0 || n_nets <= 0) return fail(HC_E_INVALID, "ensemble needs networks and outputs");
+    return launch_ensemble(n, n_out, n_nets, preds, out_std, spread_T, spread_Y, mean, spread,
+                           static_cast<cudaStream_t>(stream));
+}
 int hc_surrogate_gate(hc_mech_t m, int64_t n, double *T, const double *p, double *rho, double *Y,
                       const float *pred, const float *X, const double *out_mean,
                       const double *out_std, const double *proj, const double *elem, int nel,

@@ -24,6 +24,8 @@
 #include <vector>
 
 #include "../../include/hurchem_b200.h"
+#include "launch.cuh"
+#include "mlp_fused.cuh"
 #include "mlp_gemm.cuh"
 
 using namespace hc;
@@ -83,14 +85,20 @@ int make_tmap(CUtensorMap *tm, const void *base, uint64_t rows, uint64_t cols, u
     return HC_OK;
 }
 
-constexpr int kStages = 4;
+// Pipeline depth: four stages for a long K (the weight gradients, K = batch). A
+// layer's K is a few 64-wide blocks and its time goes to the epilogue (256
+// activations per thread and tile): two stages leave room for two blocks on an
+// SM, one's epilogue under the other's loads and MMAs (300,000 rows through
+// 256-wide layers: 2497 us against 2960 us with four stages).
+constexpr int kStages = 4, kShortStages = 2, kShortK = 512;
 
-template <int BN>
+template <int BN, int STAGES>
 int launch_bn(const CUtensorMap &ta, const CUtensorMap &tb, int M, int N, int K,
               const GemmEpilogue &ep, int *err, cudaStream_t st) {
-    auto kern = gemm_bf16_tn_kernel<BN, kStages>;
-    const size_t smem = (size_t)kStages * GemmSmem<BN>::kStage + 1024 + 256;
-    MCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto kern = gemm_bf16_tn_kernel<BN, STAGES>;
+    const size_t smem = (size_t)STAGES * GemmSmem<BN>::kStage + 1024 + 256;
+    std::string msg;
+    if (int rc = allow_smem<gemm_bf16_tn_kernel<BN, STAGES>>(msg)) return mfail(rc, msg);
     dim3 grid(M / kGemmBM, N / BN);
     kern<<<grid, 128, smem, st>>>(ta, tb, K, ep, err);
     MCUDA(cudaGetLastError());
@@ -113,11 +121,19 @@ int gemm_bf16_tn(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ld
     if (rc != HC_OK) return rc;
     rc = make_tmap(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)BN);
     if (rc != HC_OK) return rc;
+    if (K <= kShortK) {
+        switch (BN) {
+        case 256: return launch_bn<256, kShortStages>(ta, tb, M, N, K, ep, err, st);
+        case 128: return launch_bn<128, kShortStages>(ta, tb, M, N, K, ep, err, st);
+        case 64: return launch_bn<64, kShortStages>(ta, tb, M, N, K, ep, err, st);
+        default: return launch_bn<32, kShortStages>(ta, tb, M, N, K, ep, err, st);
+        }
+    }
     switch (BN) {
-    case 256: return launch_bn<256>(ta, tb, M, N, K, ep, err, st);
-    case 128: return launch_bn<128>(ta, tb, M, N, K, ep, err, st);
-    case 64: return launch_bn<64>(ta, tb, M, N, K, ep, err, st);
-    default: return launch_bn<32>(ta, tb, M, N, K, ep, err, st);
+    case 256: return launch_bn<256, kStages>(ta, tb, M, N, K, ep, err, st);
+    case 128: return launch_bn<128, kStages>(ta, tb, M, N, K, ep, err, st);
+    case 64: return launch_bn<64, kStages>(ta, tb, M, N, K, ep, err, st);
+    default: return launch_bn<32, kStages>(ta, tb, M, N, K, ep, err, st);
     }
 }
 
@@ -321,6 +337,35 @@ int forward_packed(hc_mlp_t m, int Bp, bool train, cudaStream_t st) {
         MTRY(gemm_bf16_tn(m->act[l], m->inp[l], m->Wb[l], m->inp[l], Bp, m->outp[l], m->inp[l],
                           ep, m->err, st));
     }
+    return HC_OK;
+}
+
+// the whole network in one launch where its shape allows (mlp_fused.cuh)
+bool fused_fits(hc_mlp_t m) {
+    return m->nl <= kFusedLayers && m->n_in <= 256 && m->n_out <= 256 && m->width <= 256;
+}
+
+int forward_fused(hc_mlp_t m, const float *X, int64_t B, float *Y, cudaStream_t st) {
+    FusedMlp f{};
+    f.nl = m->nl;
+    f.n_in = m->n_in;
+    f.n_out = m->n_out;
+    for (int l = 0; l < m->nl; ++l) {
+        f.bias[l] = m->b[l];
+        f.nk[l] = (m->in[l] + kGemmBK - 1) / kGemmBK;      // the padding's further blocks are zero
+        f.bn[l] = (l + 1 == m->nl) ? (m->n_out + 31) / 32 * 32 : m->outp[l];
+        MTRY(make_tmap(&f.w[l], m->Wb[l], (uint64_t)m->outp[l], (uint64_t)m->inp[l], (uint64_t)m->inp[l],
+                       (uint32_t)f.bn[l]));
+    }
+    int dev = 0, sms = 0;
+    MCUDA(cudaGetDevice(&dev));
+    MCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    std::string err;
+    if (int rc = allow_smem<mlp_fused_kernel>(err)) return mfail(rc, err);
+    const int64_t pairs = (B + 2 * kGemmBM - 1) / (2 * kGemmBM);
+    const int grid = (int)(pairs < sms ? pairs : sms);
+    mlp_fused_kernel<<<grid, kFusedThreads, FusedSmem::bytes(), st>>>(f, X, B, Y, m->err);
+    MCUDA(cudaGetLastError());
     return HC_OK;
 }
 
@@ -556,6 +601,7 @@ int hc_mlp_forward(hc_mlp_t m, const float *X, int64_t B, float *Y, void *stream
     if (B <= 0) return HC_OK;
     std::lock_guard<std::mutex> lk(m->mu);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (fused_fits(m)) return forward_fused(m, X, B, Y, st);
     for (int64_t r0 = 0; r0 < B; r0 += m->cap) {
         const int nb = (int)std::min<int64_t>(m->cap, B - r0);
         const int Bp = pad128(nb);

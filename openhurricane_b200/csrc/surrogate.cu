@@ -63,6 +63,33 @@ __global__ void features_kernel(int nsp, int64_t n, const double *__restrict__ T
 }
 
 
+// the networks' mean prediction and their disagreement, thread per cell
+__global__ void ensemble_kernel(int64_t n, int n_out, int n_nets, const float *__restrict__ preds,
+                                const double *__restrict__ out_std, double spread_T, double spread_Y,
+                                float *__restrict__ mean, float *__restrict__ spread) {
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n;
+         c += (int64_t)gridDim.x * blockDim.x) {
+        double worst = 0.0;
+        bool nan = false;
+        for (int j = 0; j < n_out; ++j) {
+            const float *p = preds + c * n_out + j;
+            float s = 0.0f, lo = INFINITY, hi = -INFINITY;
+            for (int k = 0; k < n_nets; ++k) {
+                const float v = p[k * n * n_out];
+                s += v;
+                nan = nan || isnan(v);
+                lo = fminf(lo, v);
+                hi = fmaxf(hi, v);
+            }
+            mean[c * n_out + j] = s / (float)n_nets;
+            const double r = (double)(hi - lo) * out_std[j] / (j == 0 ? spread_T : spread_Y);
+            nan = nan || isnan(r);               // equal infinities
+            worst = r > worst ? r : worst;
+        }
+        spread[c] = nan ? NAN : (float)worst;
+    }
+}
+
 __global__ void gate_kernel(const __grid_constant__ DevMech m, const __grid_constant__ GateArgs a) {
     const int nsp = m.nsp;
     const int n_in = nsp + 3, n_out = nsp + 1;
@@ -198,6 +225,19 @@ __global__ void gate_kernel(const __grid_constant__ DevMech m, const __grid_cons
             a.rejected[slot] = (int32_t)c;
         }
     }
+}
+
+int launch_ensemble(int64_t n, int n_out, int n_nets, const float *preds, const double *out_std, double spread_T,
+                    double spread_Y, float *mean, float *spread, cudaStream_t st) {
+    const int64_t blocks = (n + 127) / 128;
+    ensemble_kernel<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 128, 0, st>>>(
+        n, n_out, n_nets, preds, out_std, spread_T, spread_Y, mean, spread);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) {
+        set_last_error(std::string("ensemble kernel: ") + cudaGetErrorString(e));
+        return HC_E_CUDA;
+    }
+    return HC_OK;
 }
 
 int launch_features(const DevMech &m, int64_t n, const double *T, const double *p,

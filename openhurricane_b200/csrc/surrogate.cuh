@@ -34,6 +34,8 @@ struct GateArgs {
 int launch_features(const DevMech &m, int64_t n, const double *T, const double *p,
                     const double *Y, const double *dt, double dt_factor, const double *mean,
                     const double *inv_std, float *X, cudaStream_t st);
+int launch_ensemble(int64_t n, int n_out, int n_nets, const float *preds, const double *out_std, double spread_T,
+                    double spread_Y, float *mean, float *spread, cudaStream_t st);
 int launch_gate(const DevMech &m, const GateArgs &a, cudaStream_t st);
 
 }  // namespace hc

@@ -228,13 +228,18 @@ class Surrogate:
         """Mean normalised prediction of the ensemble and its per-cell
         disagreement (the larger of the dT spread / spread_T and the largest
         dY spread / spread_Y; <= 1 is confident)."""
-        preds = torch.stack([net.forward(X) for net in self.nets])
-        mean = preds.mean(dim=0).contiguous()
         if len(self.nets) == 1:
-            return mean, None
-        rng = (preds.max(dim=0).values - preds.min(dim=0).values).double() * self.out_std[None, :]
-        sp = torch.maximum(rng[:, 0] / self.spread_T, rng[:, 1:].max(dim=1).values / self.spread_Y)
-        return mean, sp.to(torch.float32).contiguous()
+            return self.nets[0].forward(X), None
+        n = int(X.shape[0])
+        preds = torch.empty((len(self.nets), n, self.n_out), dtype=torch.float32, device=X.device)
+        for k, net in enumerate(self.nets):
+            net.forward(X, out=preds[k])
+        mean = torch.empty((n, self.n_out), dtype=torch.float32, device=X.device)
+        spread = torch.empty(n, dtype=torch.float32, device=X.device)
+        _capi.check(_capi.load().hc_surrogate_ensemble(
+            n, self.n_out, len(self.nets), _vp(preds), _vp(self.out_std), float(self.spread_T),
+            float(self.spread_Y), _vp(mean), _vp(spread), _vp_stream()), "hc_surrogate_ensemble")
+        return mean, spread
 
     # ------------------------------------------------------------------ infer
     def step(self, flow, dt: torch.Tensor, dt_factor: float = 1.0, opts=None,

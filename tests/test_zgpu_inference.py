@@ -1,0 +1,84 @@
+"""The network's inference kernel and the ensemble kernel on the GPU: the
+fused forward pass at the edges of its tiles and shapes (and the layer-by-layer
+one just past them) against the same network in float64 on the operands the
+kernel multiplies, the ensemble's mean and spread against the same formulas."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev():
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    return torch.device("cuda:0")
+
+
+def _reference(theta, shapes, X):
+    """float64, with the input, the weights and every activation rounded to BF16
+    as the kernels round them; also a bound on what one more BF16 rounding of the
+    activations (a value next to a rounding boundary) can change."""
+    bf = lambda a: torch.as_tensor(a, dtype=torch.float32).to(torch.bfloat16).double()
+    h, err, off = bf(X), None, 0
+    for l, (o, i) in enumerate(shapes):
+        W = bf(theta[off:off + o * i].reshape(o, i))
+        b = torch.as_tensor(theta[off + o * i:off + o * i + o]).double()
+        off += o * i + o
+        # fp32 accumulation of i products, and the error carried in
+        a = h.abs() @ W.abs().T + b.abs()
+        err = a * (i + 2) * 2.0 ** -24 + (0.0 if err is None else err @ W.abs().T)
+        h = h @ W.T + b
+        if l + 1 < len(shapes):
+            h = torch.nn.functional.gelu(h)
+            err = 1.13 * err + 2e-7                  # |gelu'| < 1.13, the approximation of erf
+            h, err = bf(h.float()), err + h.abs() * 2.0 ** -8
+    return h, err
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 64), (12, 10, 3, 256), (56, 54, 2, 256), (64, 64, 1, 128),
+                                   (65, 65, 2, 192), (256, 256, 1, 256), (12, 10, 2, 320)])
+@pytest.mark.parametrize("B", [1, 127, 128, 129, 2000])
+def test_forward_matches_float64_on_rounded_operands(shape, B):
+    from openhurricane_b200.surrogate import MLP
+    dev = _dev()
+    n_in, n_out, nh, w = shape
+    net = MLP(n_in, n_out, nh, w, max_batch=1024, seed=5)
+    X = np.random.default_rng(B).normal(size=(B, n_in)).astype(np.float32)
+    out = net.forward(torch.tensor(X, device=dev)).cpu().double()
+    ref, err = _reference(net.get_params(), net.shapes(), X)
+    assert out.shape == ref.shape
+    assert torch.all((out - ref).abs() <= err), ((out - ref).abs() / err).max()
+
+
+@pytest.mark.parametrize("n,n_out,n_nets", [(1, 1, 1), (257, 10, 2), (4096, 54, 4), (1000, 7, 3)])
+def test_ensemble_matches_its_formulas(n, n_out, n_nets):
+    import ctypes as C
+    from openhurricane_b200 import _capi
+    dev = _dev()
+    rng = np.random.default_rng(n)
+    P = rng.normal(size=(n_nets, n, n_out)).astype(np.float32)
+    if n > 1:
+        P[n_nets - 1, n // 2, n_out - 1] = np.nan
+        P[0, n // 3, 0] = np.inf
+        P[:, 0, 0] = -np.inf
+    scale = rng.uniform(0.5, 2.0, n_out)
+    p, s = torch.tensor(P, device=dev), torch.tensor(scale, device=dev)
+    mean = torch.empty(n, n_out, dtype=torch.float32, device=dev)
+    spread = torch.empty(n, dtype=torch.float32, device=dev)
+    vp = lambda t: C.c_void_p(t.data_ptr())
+    _capi.check(_capi.load().hc_surrogate_ensemble(n, n_out, n_nets, vp(p), vp(s), 50.0, 1e-2, vp(mean), vp(spread),
+                                                   C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+                "hc_surrogate_ensemble")
+    with np.errstate(invalid="ignore"):
+        Q = P.astype(np.float64)
+        m = Q.mean(axis=0)
+        d = (Q.max(axis=0) - Q.min(axis=0)) * scale / np.where(np.arange(n_out) == 0, 50.0, 1e-2)
+        sp = d.max(axis=1)                           # NaN where a prediction is NaN
+    # at most n_nets + 1 float32 roundings of values up to the largest magnitude
+    tol = (n_nets + 1) * 2.0 ** -23 * np.nanmax(np.where(np.isfinite(Q), np.abs(Q), 0.0))
+    got = mean.cpu().numpy()
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(m))
+    np.testing.assert_allclose(got, m, rtol=0.0, atol=tol)
+    np.testing.assert_allclose(spread.cpu().numpy(), sp, rtol=4 * 2.0 ** -23, atol=1e-4)
