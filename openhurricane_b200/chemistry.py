@@ -24,13 +24,17 @@ from . import _capi
 from .mechanism import MechTables, compile_mechanism
 
 
+# A call's arguments as plain integers: every signature of _capi declares its
+# pointers, so ctypes converts them, and a small call (a few microseconds on the
+# device) is not spent on building c_void_p and Stream objects.
 def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _stream(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _f64(t: torch.Tensor, name: str) -> torch.Tensor:
@@ -58,7 +62,8 @@ class Mechanism:
         return cls(compile_mechanism(che, thermo, transport))
 
     def set_tuning(self, kernel: int = 0, block: int = 64):
-        """kernel: 0 automatic (warp per cell where it applies, else the cell group),
+        """kernel: 0 automatic (warp per cell up to 16 unknowns, block per cell above, the cell
+        group where these do not apply),
         1 table-driven thread per cell, 2 cell group,
         3 generated thread per cell, 4 compact thread per cell, 5 generated direct-assembly
         thread per cell, 6 warp per cell, 7 segment per cell (see hc_set_tuning)."""
