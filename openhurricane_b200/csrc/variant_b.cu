@@ -24,11 +24,11 @@ bool launch_b_fits(const RMech &m, const BMech &b) {
     return N <= 64 && HC_B_DISPATCH(N, b_smem, m, b) <= kMaxSmem;
 }
 
-template <class K>
-static int b_grid(K kern, size_t sm, int num_sms, int64_t n, int64_t &grid, std::string &err) {
+template <auto Kernel>
+static int b_grid(size_t sm, int num_sms, int64_t n, int64_t &grid, std::string &err) {
     int per_sm = 0;
-    HC_LCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBThreads, sm));
+    if (int rc = allow_smem<Kernel>(err)) return rc;
+    HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Kernel, kBThreads, sm));
     if (per_sm < 1) {
         err = "block-per-cell kernel does not fit on an SM";
         return HC_E_UNSUPPORTED;
@@ -40,12 +40,11 @@ static int b_grid(K kern, size_t sm, int num_sms, int64_t n, int64_t &grid, std:
 template <int CPW, int SL>
 static int launch_bi(const RMech &m, const BMech &b, int num_sms, const IntegratorParams &P, const CellIO &io,
                      cudaStream_t st, std::string &err) {
-    auto kern = integrate_b_kernel<CPW, SL>;
     const size_t sm = b_smem<CPW, SL>(m, b);
     int64_t grid = 0;
-    const int rc = b_grid(kern, sm, num_sms, io.nqueue, grid, err);
+    const int rc = b_grid<integrate_b_kernel<CPW, SL>>(sm, num_sms, io.nqueue, grid, err);
     if (rc != HC_OK || grid <= 0) return rc;
-    kern<<<(unsigned)grid, kBThreads, sm, st>>>(m, b, P, io);
+    integrate_b_kernel<CPW, SL><<<(unsigned)grid, kBThreads, sm, st>>>(m, b, P, io);
     HC_LCUDA(cudaGetLastError());
     return HC_OK;
 }
@@ -58,13 +57,12 @@ int launch_integrate_b(const RMech &m, const BMech &b, int num_sms, const Integr
 template <int CPW, int SL>
 static int launch_bj(const RMech &m, const BMech &b, int num_sms, int64_t n, const double *c, const double *T,
                      double *dydt, double *J, cudaStream_t st, std::string &err) {
-    auto kern = jacobian_b_kernel<CPW, SL>;
     const size_t sm = b_smem<CPW, SL>(m, b);
     int64_t grid = 0;
-    const int rc = b_grid(kern, sm, num_sms, n, grid, err);
+    const int rc = b_grid<jacobian_b_kernel<CPW, SL>>(sm, num_sms, n, grid, err);
     if (rc != HC_OK || grid <= 0) return rc;
     IntegratorParams P{};
-    kern<<<(unsigned)grid, kBThreads, sm, st>>>(m, b, P, n, c, T, dydt, J);
+    jacobian_b_kernel<CPW, SL><<<(unsigned)grid, kBThreads, sm, st>>>(m, b, P, n, c, T, dydt, J);
     HC_LCUDA(cudaGetLastError());
     return HC_OK;
 }

@@ -76,9 +76,11 @@ static int launch_s(const WMech &m, int num_sms, const IntegratorParams &P, cons
     constexpr int G = SLayout<N>::G;
     const size_t sm = w_tables_bytes(m.nsp, m.nrc, m.nrc32, m.nent, m.ntb, m.njob32) +
                       sizeof(double) * SLayout<N>::doubles(m.nrc, m.njob) * G * kSWarps;
-    HC_LCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     int per_sm = 0;
-    HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kSWarps, sm));
+    if (sm <= kMaxSmem) {
+        if (int rc = allow_smem<integrate_s_kernel<N>>(err)) return rc;
+            HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kSWarps, sm));
+    }
     if (per_sm < 1) {
         err = "segment-per-cell kernel does not fit on an SM";
         return HC_E_UNSUPPORTED;
