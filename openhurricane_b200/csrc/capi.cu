@@ -54,19 +54,40 @@ int fail(int code, const std::string &msg) {
             return fail(HC_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-template <typename T>
-int upload(std::vector<void *> &owned, const T *src, size_t n, const T **dst) {
-    if (n == 0) {
+// A handle's device tables: gathered on the host, then one allocation and one copy (an
+// allocation and a copy for each of the 40 to 60 tables was most of a handle's creation)
+class Tables {
+public:
+    template <typename T>
+    void add(const T *src, size_t n, const T **dst) {
         *dst = nullptr;
+        if (n == 0) return;
+        const size_t at = (bytes_.size() + 255) & ~(size_t)255;
+        bytes_.resize(at + n * sizeof(T));
+        std::memcpy(bytes_.data() + at, src, n * sizeof(T));
+        places_.push_back({dst, at});
+    }
+    int upload(std::vector<void *> &owned) {
+        if (bytes_.empty()) return HC_OK;
+        void *d = nullptr;
+        HC_CUDA(cudaMalloc(&d, bytes_.size()));
+        owned.push_back(d);
+        HC_CUDA(cudaMemcpy(d, bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice));
+        for (const Place &p : places_) {
+            const void *q = static_cast<char *>(d) + p.at;
+            std::memcpy(p.dst, &q, sizeof(q));
+        }
         return HC_OK;
     }
-    void *d = nullptr;
-    HC_CUDA(cudaMalloc(&d, n * sizeof(T)));
-    owned.push_back(d);
-    HC_CUDA(cudaMemcpy(d, src, n * sizeof(T), cudaMemcpyHostToDevice));
-    *dst = static_cast<const T *>(d);
-    return HC_OK;
-}
+
+private:
+    struct Place {
+        void *dst;
+        size_t at;
+    };
+    std::vector<char> bytes_;
+    std::vector<Place> places_;
+};
 
 enum Variant { kV10 = 0, kV16, kV32, kV54, kV64 };
 
@@ -486,8 +507,11 @@ static bool pack_b(const RHost &r, int nsp, BHost &o) {
             for (int k = 0; k < 32; ++k) o.task.push_back(32 * t + k < nrc ? order[32 * t + k] : -1);
         o.tptr.push_back((int)o.task.size() / 32);
     }
-    // terms: place in the records, sign
-    std::vector<std::vector<uint32_t>> item(nsp * b.ld + nsp);   // J region, then the rows' sums
+    // terms: place in the records, sign. By item (J region, then the rows' sums) in the
+    // reactions' order: counted, then written behind one another.
+    const int nitem = nsp * b.ld + nsp;
+    std::vector<std::pair<int, uint32_t>> raw;
+    raw.reserve(64 * (size_t)nrc);
     for (int q = 0; q < nrc; ++q) {
         const int4 c = r.code[q];
         int sp[6], nu[6], at[6];
@@ -498,7 +522,7 @@ static bool pack_b(const RHost &r, int nsp, BHost &o) {
             at[k] = q * b.stride + kBd + (k < 3 ? k : F + k - 3);
         }
         auto add = [&](int to, int n, int place) {
-            for (int k = 0; k < std::abs(n); ++k) item[to].push_back((uint32_t)place | (n < 0 ? 0x8000u : 0u));
+            for (int k = 0; k < std::abs(n); ++k) raw.push_back({to, (uint32_t)place | (n < 0 ? 0x8000u : 0u)});
         };
         for (int k = 0; k < 6; ++k) {
             if (sp[k] < 0) continue;
@@ -513,19 +537,28 @@ static bool pack_b(const RHost &r, int nsp, BHost &o) {
             for (int e = e0; e < e0 + ne; ++e) add(i * b.ld + r.eidx[e], nu[k], nrc * b.stride + e);
         }
     }
+    std::vector<int> first(nitem + 1, 0);
+    for (const auto &t : raw) ++first[t.first + 1];
+    for (int i = 0; i < nitem; ++i) first[i + 1] += first[i];
+    std::vector<uint32_t> terms(raw.size());
+    {
+        std::vector<int> next(first.begin(), first.end() - 1);
+        for (const auto &t : raw) terms[next[t.first]++] = t.second;
+    }
+    auto length = [&](int i) { return first[i + 1] - first[i]; };
     std::vector<int> ids;
-    for (size_t i = 0; i < item.size(); ++i)
-        if (!item[i].empty()) ids.push_back((int)i);
-    std::stable_sort(ids.begin(), ids.end(), [&](int x, int y) { return item[x].size() > item[y].size(); });
+    for (int i = 0; i < nitem; ++i)
+        if (length(i) > 0) ids.push_back(i);
+    std::stable_sort(ids.begin(), ids.end(), [&](int x, int y) { return length(x) > length(y); });
     // 64 items a pair of groups: lane l has items l and 32 + l, as long as the longest
     cost.clear();
-    for (size_t i = 0; i < ids.size(); i += 64) cost.push_back(2.0 + (item[ids[i]].size() + 1) / 2);
+    for (size_t i = 0; i < ids.size(); i += 64) cost.push_back(2.0 + (length(ids[i]) + 1) / 2);
     const uint32_t nothing = (uint32_t)zero | (uint32_t)zero << 16;
     if (nsp * b.ld >= (int)kBRow) return false;
     o.gptr.assign(1, 0);
     for (const auto &list : balance(cost)) {
         for (int g : list) {
-            const int words = ((int)item[ids[64 * (size_t)g]].size() + 1) / 2, base = (int)o.term.size() / 32;
+            const int words = (length(ids[64 * (size_t)g]) + 1) / 2, base = (int)o.term.size() / 32;
             if (base >= (1 << 16) || words >= (1 << 15)) return false;
             o.term.resize(o.term.size() + 32 * (size_t)words, make_uint2(nothing, nothing));
             for (int l = 0; l < 32; ++l) {
@@ -536,10 +569,11 @@ static bool pack_b(const RHost &r, int nsp, BHost &o) {
                     if (at >= ids.size()) continue;
                     const int id = ids[at];
                     to[half] = id < nsp * b.ld ? (uint32_t)id : kBRow | (uint32_t)(id - nsp * b.ld);
-                    for (size_t k = 0; k < item[id].size(); ++k) {
-                        uint2 &v = o.term[32 * (size_t)(base + (int)k / 2) + l];
+                    const uint32_t *item = &terms[first[id]];
+                    for (int k = 0; k < length(id); ++k) {
+                        uint2 &v = o.term[32 * (size_t)(base + k / 2) + l];
                         uint32_t &w = half ? v.y : v.x;
-                        w = (k & 1) ? (w & 0xffffu) | item[id][k] << 16 : (w & 0xffff0000u) | item[id][k];
+                        w = (k & 1) ? (w & 0xffffu) | item[k] << 16 : (w & 0xffff0000u) | item[k];
                     }
                 }
                 o.dst.push_back(to[0] | to[1] << 16);
@@ -884,10 +918,8 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
     dm.nsp = nsp;
     dm.nrc = nrc;
     dm.ext = hm.ext ? 1 : 0;
-    int rc = HC_OK;
-    auto up = [&](auto *src, size_t n, auto **dst) {
-        if (rc == HC_OK) rc = upload(m->owned, src, n, dst);
-    };
+    Tables tables;
+    auto up = [&](auto *src, size_t n, auto **dst) { tables.add(src, n, dst); };
     up(d->W, nsp, &dm.W);
     up(d->Trange, 3 * (size_t)nsp, &dm.Trange);
     up(d->nasa, 14 * (size_t)nsp, &dm.nasa);
@@ -934,7 +966,7 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
             up(wh.gslot.data(), wh.gslot.size(), &w.gslot);
             up(wh.gnu.data(), wh.gnu.size(), &w.gnu);
             up(wh.raw.data(), wh.raw.size(), &w.raw);
-            m->w_ok = (rc == HC_OK);
+            m->w_ok = true;
         }
     }
     {
@@ -949,9 +981,10 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
             up(rh.eidx.data(), rh.eidx.size(), &r.eidx);
             up(rh.eval.data(), rh.eval.size(), &r.eval);
             up(rh.fall.data(), rh.fall.size(), &r.fall);
-            m->r_ok = (rc == HC_OK);
+            m->r_ok = true;
             BHost bh;
-            if (pack_b(rh, hm.nsp, bh)) {
+            // up to 16 unknowns nothing reads them
+            if (nsp + 1 > 16 && pack_b(rh, hm.nsp, bh)) {
                 BMech &b = m->b;
                 b = bh.b;
                 up(bh.task.data(), bh.task.size(), &b.task);
@@ -960,7 +993,7 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
                 up(bh.pair.data(), bh.pair.size(), &b.pair);
                 up(bh.dst.data(), bh.dst.size(), &b.dst);
                 up(bh.term.data(), bh.term.size(), &b.term);
-                m->b_ok = (rc == HC_OK) && launch_b_fits(m->r, b);
+                m->b_ok = launch_b_fits(m->r, b);
             }
         }
     }
@@ -1010,6 +1043,7 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
         }
         up(t.data(), t.size(), &dm.ptab);
     }
+    int rc = tables.upload(m->owned);
     if (rc == HC_OK) {
         void *q = nullptr;
         cudaError_t e = cudaMalloc(&q, 8 * sizeof(unsigned long long));

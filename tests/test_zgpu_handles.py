@@ -113,3 +113,44 @@ def test_jacobians_of_two_mechanisms_in_two_threads(loops, tmp_path):
     _all_at_once(jobs)
     for h in held:
         h[0].close()
+
+
+@pytest.mark.parametrize("name,pairs", [("small", 30), ("large", 45)])
+def test_creating_a_handle_takes_few_allocations(name, pairs, request):
+    """The device tables come in one allocation and one copy. The bar is the time of that many
+    allocations and copies; with one for each table a handle took over 60 and the packing
+    of the tables (the large mechanism's is half of what it takes now)."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    from openhurricane_b200 import _capi
+    _dev()
+    tables = request.getfixturevalue(name)["tables"]
+    lib = _capi.load()
+    desc = _capi.DescArrays(tables)
+    part = np.zeros(4096, np.uint8)
+    torch.cuda.synchronize()
+
+    def create():
+        h = C.c_void_p()
+        assert lib.hc_mech_create(C.byref(desc.desc), C.byref(h)) == 0
+        lib.hc_mech_destroy(h)
+
+    def allocate():
+        held = []
+        for _ in range(pairs):
+            err, q = rt.cudaMalloc(65536)
+            assert int(err) == 0
+            held.append(q)
+            rt.cudaMemcpy(q, part.ctypes.data, part.nbytes, rt.cudaMemcpyKind.cudaMemcpyHostToDevice)
+        for q in held:
+            rt.cudaFree(q)
+
+    def median(f):
+        ts = []
+        for _ in range(25):
+            t0 = time.perf_counter()
+            f()
+            ts.append(time.perf_counter() - t0)
+        return statistics.median(ts[5:])
+
+    took, bar = median(create), median(allocate)
+    assert took <= bar, (took, bar)
