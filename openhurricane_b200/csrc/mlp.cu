@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/hurchem_b200.h"
+#include "gemm_rule.h"
 #include "launch.cuh"
 #include "mlp_fused.cuh"
 #include "mlp_gemm.cuh"
@@ -85,13 +86,6 @@ int make_tmap(CUtensorMap *tm, const void *base, uint64_t rows, uint64_t cols, u
     return HC_OK;
 }
 
-// Pipeline depth: four stages for a long K (the weight gradients, K = batch). A
-// layer's K is a few 64-wide blocks and its time goes to the epilogue (256
-// activations per thread and tile): two stages leave room for two blocks on an
-// SM, one's epilogue under the other's loads and MMAs (300,000 rows through
-// 256-wide layers: 2497 us against 2960 us with four stages).
-constexpr int kStages = 4, kShortStages = 2, kShortK = 512;
-
 template <int BN, int STAGES>
 int launch_bn(const CUtensorMap &ta, const CUtensorMap &tb, int M, int N, int K,
               const GemmEpilogue &ep, int *err, cudaStream_t st) {
@@ -121,19 +115,22 @@ int gemm_bf16_tn(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ld
     if (rc != HC_OK) return rc;
     rc = make_tmap(&tb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, (uint32_t)BN);
     if (rc != HC_OK) return rc;
-    if (K <= kShortK) {
+    int dev = 0, sms = 0;
+    MCUDA(cudaGetDevice(&dev));
+    MCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (gemm_stages(M / kGemmBM, N / BN, K, sms) == kShortRing) {
         switch (BN) {
-        case 256: return launch_bn<256, kShortStages>(ta, tb, M, N, K, ep, err, st);
-        case 128: return launch_bn<128, kShortStages>(ta, tb, M, N, K, ep, err, st);
-        case 64: return launch_bn<64, kShortStages>(ta, tb, M, N, K, ep, err, st);
-        default: return launch_bn<32, kShortStages>(ta, tb, M, N, K, ep, err, st);
+        case 256: return launch_bn<256, kShortRing>(ta, tb, M, N, K, ep, err, st);
+        case 128: return launch_bn<128, kShortRing>(ta, tb, M, N, K, ep, err, st);
+        case 64: return launch_bn<64, kShortRing>(ta, tb, M, N, K, ep, err, st);
+        default: return launch_bn<32, kShortRing>(ta, tb, M, N, K, ep, err, st);
         }
     }
     switch (BN) {
-    case 256: return launch_bn<256, kStages>(ta, tb, M, N, K, ep, err, st);
-    case 128: return launch_bn<128, kStages>(ta, tb, M, N, K, ep, err, st);
-    case 64: return launch_bn<64, kStages>(ta, tb, M, N, K, ep, err, st);
-    default: return launch_bn<32, kStages>(ta, tb, M, N, K, ep, err, st);
+    case 256: return launch_bn<256, kLongRing>(ta, tb, M, N, K, ep, err, st);
+    case 128: return launch_bn<128, kLongRing>(ta, tb, M, N, K, ep, err, st);
+    case 64: return launch_bn<64, kLongRing>(ta, tb, M, N, K, ep, err, st);
+    default: return launch_bn<32, kLongRing>(ta, tb, M, N, K, ep, err, st);
     }
 }
 
