@@ -40,32 +40,33 @@ constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr int kGemmBM = 128;
 constexpr int kGemmBK = 64;
 
-// Normal CDF: Abramowitz & Stegun 7.1.26, erfc(x) = (a1 t + .. + a5 t^5) e^(-x^2)
-// with t = 1 / (1 + p x), absolute error <= 1.5e-7: 2^14 times below the bf16
-// rounding of the activations it feeds. One reciprocal, one exponential and 9
-// multiply-adds without a branch; the epilogues' erff (both of its ranges, one
-// per lane) was what the layers waited on (see gemm_bf16_tn_kernel). e returns e^(-z^2/2).
-__device__ __forceinline__ float normal_cdf(float z, float &e) {
-    const float x = fabsf(z) * 0.70710678118654752f;
-    const float t = __fdividef(1.0f, fmaf(0.3275911f, x, 1.0f));
-    e = __expf(-x * x);
-    float q = fmaf(1.061405429f, t, -1.453152027f);
-    q = fmaf(q, t, 1.421413741f);
-    q = fmaf(q, t, -0.284496736f);
-    q = fmaf(q, t, 0.254829592f);
-    q *= 0.5f * t * e;
-    return z < 0.0f ? q : 1.0f - q;
-}
-
+// GELU z Phi(z) = max(z, 0) - |z| Q(|z|), Q the upper tail of the normal distribution as
+// t P(t) e^(-z^2/2) with t = 1 / (1 + |z| / 4): one reciprocal, one exponential and nine
+// multiply-adds without a branch (erff has two ranges, one per lane, and the epilogues
+// waited on it). P is a fit of degree 6 to the exact e^(z^2/2) Q(z) / t on 0 <= z <= 14 by
+// least squares reweighted to the smallest maximum (Lawson): the absolute error of z Q(z)
+// is below 5e-9 and the relative one of Q below 5e-5, the rest is float rounding. Measured
+// (B200) against float64 on normal z and -8 .. 8, largest / root mean square error: 2.4e-7
+// / 2.3e-8, with erff 4.9e-7 / 2.5e-8; at z = -4 relative 4e-6, with erff 7e-3. Predictions of
+// 131,072 rows 471 us, with erff 522. +inf stays, -inf and NaN give NaN, as z Phi(z) does.
 __device__ __forceinline__ float gelu_f(float z) {
+    const float x = z > 16.0f ? 16.0f : fabsf(z);
+    const float t = __fdividef(1.0f, fmaf(0.25f, x, 1.0f));
     float e;
-    return z * normal_cdf(z, e);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-0.72134752f * x * x));
+    float q = fmaf(-0.0924931021f, t, 0.345545239f);
+    q = fmaf(q, t, -0.274037059f);
+    q = fmaf(q, t, 0.287664942f);
+    q = fmaf(q, t, 0.021574698f);
+    q = fmaf(q, t, 0.11300424f);
+    q = fmaf(q, t, 0.0987410383f);
+    return fmaf(-x, q * (t * e), fmaxf(z, 0.0f));
 }
 
+// its derivative Phi(z) + z phi(z), in the training gradients
 __device__ __forceinline__ float gelu_grad_f(float z) {
-    float e;
-    const float c = normal_cdf(z, e);
-    return fmaf(z * 0.39894228040143268f, e, c);
+    return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) +
+           z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
 template <int BN>

@@ -37,6 +37,31 @@ def _reference(theta, shapes, X):
     return h, err
 
 
+def test_gelu_against_float64():
+    """The epilogues' GELU of exact float32 arguments (a product with zeros, the arguments
+    as the bias): rounding of the result, a dozen float roundings of |z| Q(|z|) and the
+    fit's 5e-9; in the negative tail, where the value itself is small, the fit's 5e-5 of it
+    and the rounding of the exponent z^2 / 2."""
+    from openhurricane_b200.surrogate import gemm_bf16
+    dev = _dev()
+    rng = np.random.default_rng(0)
+    z = np.concatenate([rng.normal(size=200000), rng.uniform(-8, 8, 200000), np.linspace(-8, 8, 62141),
+                        [0.0, -0.0, 1e-30, 5e-324, 100.0, 1e30, 3e38]]).astype(np.float32)
+    z = np.concatenate([z, np.full(-len(z) % 32, 1.0, np.float32)])
+    A = torch.zeros(128, 64, dtype=torch.bfloat16, device=dev)
+    B = torch.zeros(len(z), 64, dtype=torch.bfloat16, device=dev)
+    got = gemm_bf16(A, B, torch.tensor(z, device=dev), act=1)[0].cpu().double().numpy()
+    x = z.astype(np.float64)
+    tail = 0.5 * torch.special.erfc(torch.tensor(np.abs(x) / np.sqrt(2.0))).numpy() * np.abs(x)
+    ref = np.maximum(x, 0.0) - tail
+    assert (np.abs(got - ref) <= 2.0 ** -24 * np.abs(ref) + 12 * 2.0 ** -24 * tail + 5e-9).all()
+    low = x < -3.0
+    assert (np.abs(got - ref)[low] <= (5e-5 + 2.0 ** -22 * (12.0 + x[low] ** 2)) * -ref[low]).all()
+    v = torch.tensor([np.inf, -np.inf, np.nan] + [1.0] * 29, dtype=torch.float32, device=dev)
+    got = gemm_bf16(A, B[:32], v, act=1)[0].cpu().numpy()
+    assert got[0] == np.inf and np.isnan(got[1]) and np.isnan(got[2]) and np.isfinite(got[3:]).all()
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 1, 64), (12, 10, 3, 256), (56, 54, 2, 256), (64, 64, 1, 128),
                                    (65, 65, 2, 192), (256, 256, 1, 256), (12, 10, 2, 320)])
 @pytest.mark.parametrize("B", [1, 127, 128, 129, 2000])
