@@ -923,6 +923,13 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
     up(d->W, nsp, &dm.W);
     up(d->Trange, 3 * (size_t)nsp, &dm.Trange);
     up(d->nasa, 14 * (size_t)nsp, &dm.nasa);
+    std::vector<double2> cph;
+    for (int k = 0; k < 2 * nsp; ++k) {
+        const double *a = d->nasa + 7 * k;
+        for (int j = 0; j < 6; j += 2) cph.push_back(make_double2(a[j], a[j + 1]));
+        cph.push_back(make_double2(a[2] / 3.0, a[4] / 5.0));
+    }
+    up(cph.data(), cph.size(), &dm.cph);
     up(p_type.data(), nrc, &dm.rate_type);
     up(p_rev.data(), nrc, &dm.reversible);
     up(p_arr.data(), 3 * (size_t)nrc, &dm.arr);
@@ -1021,25 +1028,27 @@ int hc_mech_create(const hc_mech_desc *d, hc_mech_t *out) {
         // property kernel's layout (DevMech::ptab)
         const int NB = (nsp + 3) / 4;
         const size_t tab = (size_t)4 * NB * nsp;
-        std::vector<double> t(3 * tab + 4 * (size_t)NB + 6 * (size_t)nsp, 0.0);
+        std::vector<double> t(3 * tab + 4 * (size_t)NB + 7 * (size_t)nsp, 0.0);
+        using X = long double;
         for (int i = 0; i < nsp; ++i) {
+            const X Wi = d->W[i], ei = d->eps_k[i], si = d->sigma[i];
             for (int j = 0; j < nsp; ++j) {
                 const size_t k = ((size_t)(i / 4) * nsp + j) * 4 + i % 4;
-                const double sij = 0.5 * (d->sigma[i] + d->sigma[j]);
-                const double pD = 1.858e-7 * std::sqrt(1.0 / d->W[i] + 1.0 / d->W[j]) / (sij * sij) * 1.01325e5;
-                t[k] = 1.0 / std::sqrt(8.0 * (1.0 + d->W[i] / d->W[j]));
+                const X Wj = d->W[j], sij = 0.5L * (si + d->sigma[j]);
+                t[k] = (double)(1.0L / std::sqrt(8.0L * (1.0L + Wi / Wj)));
                 if (j == i) continue;
-                t[tab + k] = 1.0 / pD;
-                t[2 * tab + k] = std::exp(0.145 * 0.5 * std::log(d->eps_k[i] * d->eps_k[j]));
+                t[tab + k] = (double)(sij * sij / ((X)1.858e-7 * std::sqrt(1.0L / Wi + 1.0L / Wj) * (X)kPatm));
+                t[2 * tab + k] = (double)std::exp((X)0.145 * 0.5L * std::log(ei * d->eps_k[j]));
             }
-            t[3 * tab + i] = 1.0 / std::sqrt(d->eps_k[i]);
-            double *q = &t[3 * tab + 4 * (size_t)NB + 6 * (size_t)i];
-            q[0] = 1.0 / d->eps_k[i];
-            q[1] = std::exp(0.145 * std::log(d->eps_k[i]));
-            q[2] = std::sqrt(d->W[i]) / (d->sigma[i] * d->sigma[i]);
-            q[3] = std::sqrt(std::sqrt(d->W[i]));
-            q[4] = 1.0 / d->W[i];
-            q[5] = kRu / d->W[i];
+            t[3 * tab + i] = (double)(1.0L / std::sqrt(ei));
+            double *q = &t[3 * tab + 4 * (size_t)NB + 7 * (size_t)i];
+            q[0] = (double)(1.0L / ei);
+            q[1] = (double)std::exp((X)0.145 * std::log(ei));
+            q[2] = (double)((X)2.6693e-6 * std::sqrt(Wi) / (si * si));
+            q[3] = (double)(1.0L / std::sqrt(Wi));
+            q[4] = (double)Wi;
+            q[5] = (double)(1.0L / Wi);
+            q[6] = kRu / d->W[i];
         }
         up(t.data(), t.size(), &dm.ptab);
     }

@@ -17,6 +17,9 @@ struct DevMech {
     const double *W;        // [nsp]
     const double *Trange;   // [nsp*3]
     const double *nasa;     // [nsp*14] low a0..a6, high a0..a6 (mass basis)
+    // [nsp][2][4] per range {a0, a1}, {a2, a3}, {a4, a5}, {a2 / 3, a4 / 5}: cp and h alone, with
+    // the two of the enthalpy's divisions that round
+    const double2 *cph;
     const int32_t *rate_type, *reversible;
     const double *arr, *arr0, *troe;  // [nrc*3], [nrc*3], [nrc*4]
     const double *sri, *arr_rev;      // [nrc*5] SRI a..e, [nrc*3] explicit reverse Arrhenius
@@ -42,7 +45,8 @@ struct DevMech {
     // the property kernel's tables, [row block of 4][j][4 rows] each: 1/sqrt(8 (1 + Wi/Wj)),
     // 1/(1.858e-7 sqrt(1/Wi + 1/Wj) / sigma_ij^2 * Patm) and (1/sqrt(eps_i eps_j))^-0.145,
     // the last two zero for j = i; then 1/sqrt(eps)
-    // of each row and per species 1/eps, (1/eps)^-0.145, sqrt(W)/sigma^2, W^(1/4), 1/W, Ru/W
+    // of each row and per species 1/eps, (1/eps)^-0.145, 2.6693e-6 sqrt(W)/sigma^2,
+    // 1/sqrt(W), W, 1/W, Ru/W; built in extended precision, each rounded once
     const double *ptab;
 };
 
@@ -95,13 +99,13 @@ __device__ __forceinline__ void species_cp_h(const DevMech &m, int i, double T, 
                                              double &h) {
     const double tl = ldg(&m.Trange[3 * i]), tc = ldg(&m.Trange[3 * i + 1]);
     const double th = ldg(&m.Trange[3 * i + 2]);
-    const double *a = (T < tc) ? &m.nasa[14 * i] : &m.nasa[14 * i + 7];
-    const double a0 = ldg(&a[0]), a1 = ldg(&a[1]), a2 = ldg(&a[2]), a3 = ldg(&a[3]);
-    const double a4 = ldg(&a[4]), a5 = ldg(&a[5]);
+    const double2 *q = m.cph + 8 * i + (T < tc ? 0 : 4);
+    const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
+    const double a0 = q0.x, a1 = q0.y, a2 = q1.x, a3 = q1.y, a4 = q2.x;
     const bool out = (T < tl || T > th);
     const double T0 = out ? hmin(hmax(T, tl), th) : T;
     cp = ((((a4 * T0 + a3) * T0 + a2) * T0 + a1) * T0 + a0);
-    h = ((((a4 * 0.2 * T0 + a3 * 0.25) * T0 + a2 * (1.0 / 3.0)) * T0 + a1 * 0.5) * T0 + a0) * T0 + a5;
+    h = ((((q3.y * T0 + a3 * 0.25) * T0 + q3.x) * T0 + a1 * 0.5) * T0 + a0) * T0 + q2.y;
     if (out) h += cp * (T - T0);
 }
 

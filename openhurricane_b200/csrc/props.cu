@@ -12,7 +12,7 @@
 // cell's blocks of four rows i. What bounds it is the FP64 pipe: the O(nsp^2)
 // pair loop, 12 FP64 instructions a pair, no division and no square root.
 //
-//  * Wilke: sqrt(mu_i / mu_j sqrt(W_j / W_i)) = S_i / S_j with S = sqrt(mu) / W^(1/4),
+//  * Wilke: sqrt(mu_i / mu_j sqrt(W_j / W_i)) = S_i / S_j with S = sqrt(mu / sqrt(W)),
 //    so sum_j phi_ij x_j = A_i + 2 S_i B_i + S_i^2 C_i with A, B, C the products of
 //    the constant matrix c_ij = 1 / sqrt(8 (1 + W_i / W_j)) with x, x / S and
 //    x / S^2 (all terms positive);
@@ -22,8 +22,15 @@
 //  * four rows per thread, so that x_j and 1/S_j are read once for four pairs and
 //    the tables come as 16-byte broadcast loads.
 //
+// Rounding: the constants come from the host's extended precision, quotients are corrected
+// to half an ulp (near_div), mu_i is formed again for its row instead of squaring 1 / R:
+// the errors against extended precision are those of the divisions and square roots it
+// replaced (mu of 9 species 1.58e-16, without these steps 2.18e-16), at the same time.
+// The pair sums stay one chain: partial sums of 16 columns cost 10 us for one cell (their
+// registers) and gain nothing over the former kernel, which had one chain too.
+//
 // Measured (B200, 65,536 cells of 53 species): 1911 us before (a warp per cell, a
-// division and a square root a pair), 338 us now.
+// division and a square root a pair), 270 us now.
 #include <cuda_runtime.h>
 
 #include <string>
@@ -38,7 +45,33 @@ namespace hc {
 constexpr int kPropMaxSp = 64;
 constexpr int kPropThreads = 512;   // most threads of a block
 constexpr int kPropCells = 128;     // most cells of a block
-constexpr int kPropSp = 6;          // constants per species at the end of DevMech::ptab
+constexpr int kPropSp = 7;          // constants per species at the end of DevMech::ptab
+
+// a / b from a and r, nearly 1 / b, to within little more than half an ulp, without the
+// division's slow path: b normal and not zero
+__device__ __forceinline__ double near_div(double a, double b, double r) {
+    const double q = a * r;
+    return fma(fma(-q, b, a), r, q);
+}
+
+// a sum in four chains, taken in turn: one chain of nsp / L additions rounds as often
+struct Sum4 {
+    double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
+    __device__ __forceinline__ void add(double y) {
+        const double t = a + y;
+        a = b;
+        b = c;
+        c = d;
+        d = t;
+    }
+    __device__ __forceinline__ double value() const { return (a + b) + (c + d); }
+};
+
+// viscosity of the species with constants q (kineticTheory.cpp:37-57): q[2] sqrt(T) over this
+__device__ __forceinline__ double species_omega(const double *q, double T, double Tpow) {
+    const double rt = fast_rcp(T * q[0] + 0.5);                  // 1 / (T / eps_i + 1/2)
+    return 1.147 * (Tpow * q[1]) + rt * rt;
+}
 
 __global__ void __launch_bounds__(kPropThreads, 1)
 properties_kernel(const __grid_constant__ DevMech m, int64_t n, const double *__restrict__ T_,
@@ -50,10 +83,10 @@ properties_kernel(const __grid_constant__ DevMech m, int64_t n, const double *__
     double *pc = smem_p;                        // c, 1/d, e: [row block][j][4 rows] each
     double *pi = pc + tab, *pe = pi + tab, *se = pe + tab;   // then 1/sqrt(eps) per species
     const int cl = threadIdx.x % B, l = threadIdx.x / B;
-    double *x = se + 4 * NB + cl, *R = x + nsp * B, *part = R + nsp * B;
-    for (int i = threadIdx.x; i < 3 * tab + 4 * NB; i += blockDim.x) smem_p[i] = m.ptab[i];
-    const double *sp = m.ptab + 3 * tab + 4 * NB;            // per species: kPropSp constants
-    const double muPre = 2.6693e-6, omegaPre = 1.147, omegaExp = -0.145;
+    const double *sp = se + 4 * NB;             // and kPropSp constants per species
+    double *x = se + 4 * NB + kPropSp * nsp + cl, *R = x + nsp * B, *part = R + nsp * B;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < 3 * tab + 4 * NB + kPropSp * nsp; i += blockDim.x) smem_p[i] = ldg(&m.ptab[i]);
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         __syncthreads();
         const int64_t cell0 = tile * B + cl;
@@ -61,9 +94,10 @@ properties_kernel(const __grid_constant__ DevMech m, int64_t n, const double *__
         const int64_t cell = live ? cell0 : n - 1;
         const double T = T_[cell], p = p_[cell];
         // Yi2Xi
-        double wsum = 0.0, cps = 0.0;
+        double wsum = 0.0;
+        Sum4 cps;
         for (int i = l; i < nsp; i += L) {
-            const double w = Y[(int64_t)i * n + cell] * ldg(&sp[kPropSp * i + 4]);
+            const double w = near_div(Y[(int64_t)i * n + cell], sp[kPropSp * i + 4], sp[kPropSp * i + 5]);
             x[i * B] = w;
             wsum += w;
         }
@@ -72,7 +106,9 @@ properties_kernel(const __grid_constant__ DevMech m, int64_t n, const double *__
         wsum = 0.0;
         for (int k = 0; k < L; ++k) wsum += part[k * B];
         const double Wmean = 1.0 / hmax(wsum, kVeryTiny);
-        const double sqT = sqrt(T), Tpow = fast_exp(omegaExp * fast_log(T));
+        // T^-0.145 with what the product rounds off: every coefficient of the cell has its error
+        const double sqT = sqrt(T), lT = fast_log(T), arg = -0.145 * lT, pw = fast_exp(arg);
+        const double Tpow = fma(pw, fma(-0.145, lT, -arg), pw);
         double xt = 0.0;
         for (int i = l; i < nsp; i += L) {
             const double xi = hmax(0.0, hmin(1.0, x[i * B] * Wmean));
@@ -82,21 +118,19 @@ properties_kernel(const __grid_constant__ DevMech m, int64_t n, const double *__
             double cp0, h0;
             species_cp_h(m, i, T, cp0, h0);
             if (ha && live) ha[(int64_t)i * n + cell] = h0;
-            cps += cp0 * Y[(int64_t)i * n + cell];
+            cps.add(cp0 * Y[(int64_t)i * n + cell]);
             const double *q = sp + kPropSp * i;
-            const double rt = fast_rcp(T * ldg(&q[0]) + 0.5);                  // 1 / (T / eps_i + 1/2)
-            const double om = omegaPre * (Tpow * ldg(&q[1])) + rt * rt;
-            const double mui = muPre * (ldg(&q[2]) * sqT) * fast_rcp(om);      // sqrt(W) / sigma^2
-            R[i * B] = ldg(&q[3]) * rsqrt(mui);                                // 1 / S
+            const double om = species_omega(q, T, Tpow);
+            R[i * B] = rsqrt(near_div(q[2] * sqT, om, fast_rcp(om)) * q[3]);   // 1 / S
         }
         part[(L + l) * B] = xt;
-        part[(2 * L + l) * B] = cps;
+        part[(2 * L + l) * B] = cps.value();
         __syncthreads();
         xt = 0.0;
         for (int k = 0; k < L; ++k) xt += part[(L + k) * B];
         if (xt != 1.0) {
             const double ixt = 1.0 / xt;
-            for (int i = l; i < nsp; i += L) x[i * B] *= ixt;
+            for (int i = l; i < nsp; i += L) x[i * B] = near_div(x[i * B], xt, ixt);
         }
         __syncthreads();
         // Wilke mixing (transportList::muKappa) and mixture-averaged D_i
@@ -131,39 +165,46 @@ properties_kernel(const __grid_constant__ DevMech m, int64_t n, const double *__
                     Ds[q] = fma(xj * d[q], fma(inv, inv, Tpow * e[q]), Ds[q]);
                 }
             }
+            double wm[4] = {0.0, 0.0, 0.0, 0.0}, wk[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int i = 4 * ib + q;
                 if (i >= nsp) break;
                 const double *c = sp + kPropSp * i;
-                const double Si = fast_rcp(R[i * B]), a = ldg(&c[3]) * Si;
-                const double mui = a * a, phi = A[q] + Si * (2.0 * Bs[q] + Si * Cs[q]);
+                // mu_i again, not the square of 1 / R, which would double its rounding errors
+                const double Si = fast_rcp(R[i * B]), phi = A[q] + Si * (2.0 * Bs[q] + Si * Cs[q]);
+                const double den = species_omega(c, T, Tpow) * phi;
                 double cp0, h0;
                 species_cp_h(m, i, T, cp0, h0);
-                const double xi = x[i * B], w = mui * xi * fast_rcp(phi);
-                mum += w;
-                kappam += w * (cp0 + 1.25 * ldg(&c[5]));
+                const double xi = x[i * B];
+                wm[q] = near_div(c[2] * sqT * xi, den, fast_rcp(den));
+                wk[q] = wm[q] * (cp0 + 1.25 * c[6]);
                 if (D && live) {
                     double Dim = 0.0;
-                    if (xi < 1.0 - kVeryTiny) Dim = (1.0 - xi) * scale * frcp(Ds[q]);
+                    if (xi < 1.0 - kVeryTiny)     // a lone species has Ds = 0
+                        Dim = (Ds[q] > 1e-280 && Ds[q] < 1e280)
+                                  ? near_div(1.0 - xi, Ds[q], fast_rcp(Ds[q])) * scale
+                                  : (1.0 - xi) * scale / Ds[q];
                     if (isinf(Dim)) Dim = 0.0;
                     D[(int64_t)i * n + cell] = Dim;
                 }
             }
+            mum += (wm[0] + wm[1]) + (wm[2] + wm[3]);
+            kappam += (wk[0] + wk[1]) + (wk[2] + wk[3]);
         }
         part[l * B] = mum;
         part[(L + l) * B] = kappam;
         __syncthreads();
         if (l == 0 && live) {
-            mum = kappam = cps = 0.0;
+            double mum = 0.0, kappam = 0.0, cp = 0.0;
             for (int k = 0; k < L; ++k) {
                 mum += part[k * B];
                 kappam += part[(L + k) * B];
-                cps += part[(2 * L + k) * B];
+                cp += part[(2 * L + k) * B];
             }
             if (mu) mu[cell] = mum;
             if (kappa) kappa[cell] = kappam;
-            if (cpm) cpm[cell] = cps;
+            if (cpm) cpm[cell] = cp;
         }
     }
 }
@@ -186,7 +227,7 @@ int launch_properties(const DevMech &m, int64_t n, const double *T, const double
     // the widest block that fits and leaves no SM without cells
     const int NB = (m.nsp + 3) / 4, L = std::min(4, NB);
     int B = kPropCells;
-    auto smem = [&](int b) { return sizeof(double) * (12 * (size_t)NB * m.nsp + 4 * NB + (2 * m.nsp + 3 * L) * (size_t)b); };
+    auto smem = [&](int b) { return sizeof(double) * (12 * (size_t)NB * m.nsp + 4 * NB + kPropSp * m.nsp + (2 * m.nsp + 3 * L) * (size_t)b); };
     while (B > 32 && (smem(B) > kMaxSmem || (n + B - 1) / B < sms)) B /= 2;
     const size_t sm = smem(B);
     if (int rc = allow_smem<properties_kernel>(err)) return rc;

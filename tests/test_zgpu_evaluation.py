@@ -129,3 +129,52 @@ def test_block_per_cell_integration_vs_oracle(shape, reactor, tmp_path):
     check(t, inp, g, ref, 1e-8, opts, f"{shape[0]} species, reactor {reactor}")
     assert (cs.status.cpu().numpy() == 0).all()
     m.close()
+
+
+@pytest.mark.parametrize("name", ["small", "large"])
+def test_properties_rounding_errors(name, request):
+    """Properties against extended precision: the root mean square of the relative error in
+    units u = 2^-53. A rounding's error is up to u, 0.42 u in the mean square (uniform, and a
+    value lies anywhere between two powers of 2). Per value, independent ones adding in
+    quadrature: h about 2 beside its largest term (bar 0.65), cp a sum of 5-term polynomials
+    (10: 1.4), mu 18 (sqrt T, the power of T, the collision integral, the mixture's sums:
+    1.8), kappa another 9 (2.2), D two sums and T^1.5 / p (44: 2.8), times 1 / (1 - x), which
+    the species that makes up a cell loses."""
+    from openhurricane_b200 import synth
+    from openhurricane_b200.chemistry import Mechanism
+    dev = _dev()
+    t = request.getfixturevalue(name)["tables"]
+    L = np.longdouble
+    c = synth.dirichlet_cells(t.nsp, 400, seed=11, T_range=(800.0, 2800.0), alpha=0.3)
+    T, p, Y, W, e, sg = (np.asarray(a).astype(L) for a in (c.T, c.p, c.Y, t.W[:, None], t.eps_k, t.sigma))
+    hi = T[None] >= np.asarray(t.Trange[:, 1])[:, None]
+    a = [np.where(hi, t.nasa[:, 1, k][:, None], t.nasa[:, 0, k][:, None]).astype(L) for k in range(7)]
+    cp = a[0] + T * (a[1] + T * (a[2] + T * (a[3] + T * a[4])))
+    ha = T * (a[0] + T * (a[1] / 2 + T * (a[2] / 3 + T * (a[3] / 4 + T * a[4] / 5)))) + a[5]
+    Ru = L(1.380649e-23 * 6.02214076e23 * 1e3)
+    X = Y / W
+    X /= X.sum(0)
+    Ts = T[None] / e[:, None]
+    mu = L(2.6693e-6) * np.sqrt(W * T) / (sg[:, None] ** 2 * (L(1.147) * Ts ** L(-0.145) + (Ts + L(0.5)) ** -2))
+    num, kap, D = np.zeros_like(T), np.zeros_like(T), np.empty_like(Y)
+    for i in range(t.nsp):
+        wr = W[i] / W
+        w = X[i] * mu[i] / (X * (1 + np.sqrt(mu[i] / mu) * wr ** L(-0.25)) ** 2 / np.sqrt(8 * (1 + wr))).sum(0)
+        num += w
+        kap += w * (cp[i] + L(1.25) * Ru / W[i])
+        Ts = T[None] / np.sqrt(e[i] * e)[:, None]
+        s2 = ((sg[i] + sg) / 2)[:, None] ** 2
+        q = X * s2 * (Ts ** L(-0.145) + (Ts + L(0.5)) ** -2) * p / (
+            L(1.858e-7) * T ** L(1.5) * np.sqrt(1 / W[i] + 1 / W) * L(101325.0))
+        D[i] = (1 - X[i]) / (q.sum(0) - q[i])
+    m = Mechanism(t)
+    g = m.properties(*[torch.tensor(np.ascontiguousarray(v), dtype=torch.float64, device=dev) for v in (c.T, c.p, c.Y)])
+    u, bad = 2.0 ** -53, []
+    for k, ref, bar in (("ha", ha, 0.65), ("cp", (Y * cp).sum(0), 1.4), ("mu", num, 1.8), ("kappa", kap, 2.2),
+                        ("D", D, 2.8)):
+        r = (g[k].cpu().numpy().astype(L) - ref) / (np.abs(ref) + (cp * T if k == "ha" else 0.0))
+        r = r * (1 - X) if k == "D" else r
+        rms = float(np.sqrt((r ** 2).mean()))
+        bad = bad + [(k, rms / u)] if rms > bar * u else bad
+    m.close()
+    assert not bad, bad
