@@ -146,6 +146,7 @@ __device__ __forceinline__ RxnVals rxn_eval(const RMech &m, const int4 w, const 
             const double *fl = m.fall + (w.w >> 16) * kRFall;
             const double b0 = ldg(&fl[1]), Ta0 = ldg(&fl[2]);
             const double k0 = ldg(&fl[0]) * ex(b0 * logT - Ta0 * invT);
+            const double up = (fabs(kx) < 1e-290) ? 0x1p200 : 1.0;   // frcp takes no subnormal kx
             const bool troe = type != kLindemann;
             double e1 = 0.0, e2 = 0.0, e3 = 0.0, iT3 = 0.0, iT1 = 0.0, T2 = 0.0;
             if (troe) {
@@ -156,7 +157,7 @@ __device__ __forceinline__ RxnVals rxn_eval(const RMech &m, const int4 w, const 
                 e2 = ex(-T * iT1);
                 if (type == kTroe4) e3 = ex(-T2 * invT);
             }
-            fo = fall_off<JAC>(troe, ldg(&fl[3]), iT3, iT1, T2, e1, e2, e3, k0 * frcp(notZeroD(kx)), M,
+            fo = fall_off<JAC>(troe, ldg(&fl[3]), iT3, iT1, T2, e1, e2, e3, (k0 * up) * frcp(notZeroD(kx) * up), M,
                                (b0 + Ta0 * invT) * invT - tk, invT);
             kf = kx * fo.w;
         }
@@ -165,9 +166,10 @@ __device__ __forceinline__ RxnVals rxn_eval(const RMech &m, const int4 w, const 
     // products in the reference's order: net rates are small differences near equilibrium
     o.q = ((kf * u0) * u1) * u2 - ((kr * v0) * v1) * v2;
     if (JAC) {
-        const double pf = (u0 * u1) * u2, pb = (v0 * v1) * v2;
+        // in this order too: a product of concentrations alone underflows where the large
+        // reverse rate at low T brings it back
         const double dkf = kf * tk;
-        o.dq = pf * dkf - pb * (dkf * ra - kf * rb);
+        o.dq = ((dkf * u0) * u1) * u2 - (((dkf * ra - kf * rb) * v0) * v1) * v2;
         if (!finite(o.dq)) o.dq = 0.0;
         o.g = 0.0;
         if (type == kThirdBody) {
@@ -178,12 +180,12 @@ __device__ __forceinline__ RxnVals rxn_eval(const RMech &m, const int4 w, const 
             o.dq += finite(dT) ? dT : 0.0;
         }
         const int mf = (w.z >> kRmf) & 3, mb = (w.z >> kRmb) & 3;
-        o.d[0] = ((mf == 1) ? 1.0 : (mf == 2) ? 2.0 : 3.0) * (kf * (u1 * u2));
-        o.d[1] = kf * (u0 * u2);
-        o.d[2] = kf * (u0 * u1);
-        o.d[3] = ((mb == 1) ? -1.0 : (mb == 2) ? -2.0 : -3.0) * (kr * (v1 * v2));
-        o.d[4] = -kr * (v0 * v2);
-        o.d[5] = -kr * (v0 * v1);
+        o.d[0] = ((mf == 1) ? 1.0 : (mf == 2) ? 2.0 : 3.0) * ((kf * u1) * u2);
+        o.d[1] = (kf * u0) * u2;
+        o.d[2] = (kf * u0) * u1;
+        o.d[3] = ((mb == 1) ? -1.0 : (mb == 2) ? -2.0 : -3.0) * ((kr * v1) * v2);
+        o.d[4] = -(kr * v0) * v2;
+        o.d[5] = -(kr * v0) * v1;
     }
     return o;
 }

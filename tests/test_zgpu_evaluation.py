@@ -178,3 +178,38 @@ def test_properties_rounding_errors(name, request):
         bad = bad + [(k, rms / u)] if rms > bar * u else bad
     m.close()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("name", ["small", "large"])
+def test_rate_constants_and_concentrations_near_underflow(name, request):
+    """A fall-off reaction whose high-pressure rate lies below the normal range (its
+    reciprocal is needed for the reduced pressure), and concentrations whose products
+    underflow unless the large reverse rates of a low temperature come first."""
+    import dataclasses
+    from openhurricane_b200.chemistry import Mechanism
+    from oracle import port, srcimp_oracle
+    dev = _dev()
+    d = lambda a: torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device=dev)
+    t = request.getfixturevalue(name)["tables"]
+    arr, arr0 = t.arr.copy(), t.arr0.copy()
+    for r in np.nonzero(t.rate_type >= 2)[0]:
+        arr[r] = (1e15, 0.0, 300.0 * (np.log(1e15) + 714.0))       # 1e-310 at 300 K
+        arr0[r] = (1e20, 0.0, 0.98 * arr[r, 2])
+    for t, T, scale in ((dataclasses.replace(t, arr=arr, arr0=arr0), (299.0, 303.0), 1.0), (t, (55.0, 65.0), 1e-200)):
+        c, rho = _states(t, 65)
+        c.T[:] = np.linspace(*T, 65)
+        rho = rho * scale
+        m = Mechanism(t)
+        ref = srcimp_oracle.srcimp(t, c.T, c.p, rho, c.Y)
+        assert np.isfinite(ref["Ri"]).all() and np.isfinite(ref["diag"]).all()
+        args = d(c.T), d(c.p), d(rho), d(c.Y)
+        _close(m.source_terms(*args), ref["Ri"], 1e-11, 0, "source")
+        Ri, diag = m.source_terms_imp(*args)
+        _close(Ri, ref["Ri"], 1e-11, 0, "implicit Ri")
+        _close(diag, ref["diag"], 1e-11, 0, "diag")
+        conc = rho[None] * c.Y / t.W[:, None]
+        f, J = port.rhs_jac(port.MechDesc(t), conc, c.T, c.p)
+        gf, gJ = m.rhs_jacobian(d(conc), args[0], args[1])
+        _close(gf[:, :t.nsp], f[:, :t.nsp], 1e-11, 1, "f")
+        _close(gJ[:, :t.nsp], J[:, :t.nsp], 1e-11, 2, "J")
+        m.close()
