@@ -16,25 +16,32 @@ def _dev():
     return torch.device("cuda:0")
 
 
-def _reference(theta, shapes, X):
-    """float64, with the input, the weights and every activation rounded to BF16
-    as the kernels round them; also a bound on what one more BF16 rounding of the
-    activations (a value next to a rounding boundary) can change."""
+def _reference(theta, shapes, X, wrong=None):
+    """float64, with the input, the weights and every activation rounded to BF16 as the
+    kernels round them; also the expected square of the kernels' distance from it. That has
+    two sources, which add in quadrature over the products of a layer: float32 accumulation
+    (a few 2^-24 of the sum of magnitudes) and activations next to a boundary of BF16, which
+    round the other way: with an error s before the rounding that is a step u = 2^-8 |h| in
+    0.8 s / u of the cases. `wrong`: the same network with a mistake in it."""
     bf = lambda a: torch.as_tensor(a, dtype=torch.float32).to(torch.bfloat16).double()
-    h, err, off = bf(X), None, 0
+    h, var, off = bf(X), 0.0, 0
     for l, (o, i) in enumerate(shapes):
         W = bf(theta[off:off + o * i].reshape(o, i))
         b = torch.as_tensor(theta[off + o * i:off + o * i + o]).double()
         off += o * i + o
-        # fp32 accumulation of i products, and the error carried in
-        a = h.abs() @ W.abs().T + b.abs()
-        err = a * (i + 2) * 2.0 ** -24 + (0.0 if err is None else err @ W.abs().T)
-        h = h @ W.T + b
-        if l + 1 < len(shapes):
-            h = torch.nn.functional.gelu(h)
-            err = 1.13 * err + 2e-7                  # |gelu'| < 1.13, the approximation of erf
-            h, err = bf(h.float()), err + h.abs() * 2.0 ** -8
-    return h, err
+        last = l + 1 == len(shapes)
+        carried = var @ (W ** 2).T if l else 0.0
+        s2 = carried + ((h.abs() @ W.abs().T + b.abs()) * 2.0 ** -23) ** 2
+        if wrong == "K block" and last:
+            W = torch.cat([torch.zeros_like(W[:, :16]), W[:, 16:]], 1)
+        h = h @ W.T + (0.0 if wrong == "bias" else b)
+        var = s2
+        if not last:
+            h = torch.relu(h) if wrong == "ReLU" else torch.nn.functional.gelu(h)
+            s = 1.13 * s2.sqrt() + 1e-7              # |gelu'| < 1.13, the error of gelu_f
+            var = 0.8 * s * h.abs() * 2.0 ** -8 + s ** 2
+            h = bf(h.float())
+    return (torch.zeros_like(h) if wrong == "zero" else h), var
 
 
 def test_gelu_against_float64():
@@ -72,9 +79,16 @@ def test_forward_matches_float64_on_rounded_operands(shape, B):
     net = MLP(n_in, n_out, nh, w, max_batch=1024, seed=5)
     X = np.random.default_rng(B).normal(size=(B, n_in)).astype(np.float32)
     out = net.forward(torch.tensor(X, device=dev)).cpu().double()
-    ref, err = _reference(net.get_params(), net.shapes(), X)
+    args = net.get_params(), net.shapes(), X
+    ref, var = _reference(*args)
     assert out.shape == ref.shape
-    assert torch.all((out - ref).abs() <= err), ((out - ref).abs() / err).max()
+    rms = lambda d: float((d ** 2).mean().sqrt())
+    bar = 6.0 * float(var.mean().sqrt())
+    assert rms(out - ref) <= bar, (rms(out - ref), bar)
+    if B >= 127:
+        # the bar tells a missing bias, K slice or activation from rounding
+        for wrong in ("zero", "bias", "K block", "ReLU"):
+            assert rms(_reference(*args, wrong)[0] - ref) > 10 * bar, wrong
 
 
 @pytest.mark.parametrize("n,n_out,n_nets", [(1, 1, 1), (257, 10, 2), (4096, 54, 4), (1000, 7, 3)])
