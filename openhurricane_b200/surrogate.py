@@ -231,13 +231,20 @@ class Surrogate:
         if len(self.nets) == 1:
             return self.nets[0].forward(X), None
         n = int(X.shape[0])
+        std = self.out_std
+        if std.device != X.device:
+            raise ValueError("out_std and X are on different devices")
+        # the kernel reads n_out consecutive doubles
+        std = std.to(torch.float64).expand(self.n_out).contiguous()
+        if any(net.n_out != self.n_out for net in self.nets):
+            raise ValueError("the networks' outputs differ in number")
         preds = torch.empty((len(self.nets), n, self.n_out), dtype=torch.float32, device=X.device)
         for k, net in enumerate(self.nets):
             net.forward(X, out=preds[k])
         mean = torch.empty((n, self.n_out), dtype=torch.float32, device=X.device)
         spread = torch.empty(n, dtype=torch.float32, device=X.device)
         _capi.check(_capi.load().hc_surrogate_ensemble(
-            n, self.n_out, len(self.nets), _vp(preds), _vp(self.out_std), float(self.spread_T),
+            n, self.n_out, len(self.nets), _vp(preds), _vp(std), float(self.spread_T),
             float(self.spread_Y), _vp(mean), _vp(spread), _vp_stream()), "hc_surrogate_ensemble")
         return mean, spread
 

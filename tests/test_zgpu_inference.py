@@ -121,3 +121,34 @@ def test_ensemble_matches_its_formulas(n, n_out, n_nets):
     np.testing.assert_array_equal(np.isnan(got), np.isnan(m))
     np.testing.assert_allclose(got, m, rtol=0.0, atol=tol)
     np.testing.assert_allclose(spread.cpu().numpy(), sp, rtol=4 * 2.0 ** -23, atol=1e-4)
+
+
+def test_predict_takes_the_scales_of_any_form(small):
+    """out_std as float32, one number or every other element of a tensor gives what the
+    same values as consecutive doubles give (the kernel reads those); a scale on another
+    device and networks of other widths are refused."""
+    from openhurricane_b200.chemistry import Mechanism
+    from openhurricane_b200.surrogate import MLP, Surrogate
+    dev = _dev()
+    sur = Surrogate(Mechanism(small["tables"]), n_hidden=1, width=64, max_batch=256, seed=1)
+    X = torch.randn(100, sur.n_in, device=dev)
+    base = torch.linspace(0.5, 2.0, sur.n_out, device=dev).float()
+    spaced = torch.full((sur.n_out, 2), 7.0, dtype=torch.float64, device=dev)
+    spaced[:, 0] = base.double()
+    sur.out_std = base.double()
+    mean, spread = sur.predict(X)
+    for form in (base, spaced[:, 0]):
+        sur.out_std = form
+        m, s = sur.predict(X)
+        assert torch.equal(m, mean) and torch.equal(s, spread)
+    sur.out_std = torch.full((sur.n_out,), 0.25, dtype=torch.float64, device=dev)
+    _, spread = sur.predict(X)
+    sur.out_std = torch.tensor([0.25], dtype=torch.float64, device=dev)
+    assert torch.equal(sur.predict(X)[1], spread)
+    sur.out_std = base.double().cpu()
+    with pytest.raises(ValueError):
+        sur.predict(X)
+    sur.out_std = base.double()
+    sur.nets[1] = MLP(sur.n_in, sur.n_out + 3, 1, 64, max_batch=256)
+    with pytest.raises(ValueError):
+        sur.predict(X)
