@@ -53,7 +53,8 @@ mlp_fused_kernel(const __grid_constant__ FusedMlp net, const float *__restrict__
     uint8_t *ring = smem + 2 * S::kA;
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + kFusedRing * S::kB);
     uint64_t *empty = full + kFusedRing, *ready = empty + kFusedRing, *done = ready + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 2);
+    uint64_t *drain = done + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *stop = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t tiles = (rows + kGemmBM - 1) / kGemmBM;
@@ -68,6 +69,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMlp net, const float *__restrict__
             sm100::mbar_init(&ready[s], 128);
             sm100::mbar_init(&done[s], 1);
         }
+        sm100::mbar_init(drain, 1);
         *stop = 0;
         sm100::fence_mbar_init();
     }
@@ -107,6 +109,9 @@ mlp_fused_kernel(const __grid_constant__ FusedMlp net, const float *__restrict__
                         sm100::tma_load_2d(ring + st * S::kB, &net.w[l], &full[st], k * kGemmBK, 0);
                     }
                 }
+        // where a role gave up, loads may still be on their way into this block's memory
+        for (uint32_t i = q < kFusedRing ? 0 : q - kFusedRing; i < q; ++i)
+            sm100::mbar_wait(&full[i % kFusedRing], (i / kFusedRing) & 1, kWaitLimit);
     } else if (warp == 1 && lane == 0) {
         uint32_t q = 0, phase[2] = {0, 0};
         bool ok = true;
@@ -138,6 +143,9 @@ mlp_fused_kernel(const __grid_constant__ FusedMlp net, const float *__restrict__
                     }
                     if (ok) sm100::mma_commit(&done[s]);
                 }
+        // and MMAs into the tensor memory that is freed below
+        sm100::mma_commit(drain);
+        sm100::mbar_wait(drain, 0, kWaitLimit);
     } else if (warp >= 2) {
         const int s = (warp - 2) >> 2, quarter = warp & 3;    // the lanes of tensor memory a warp can read
         const int r = quarter * 32 + lane;                    // the thread's row of the tile

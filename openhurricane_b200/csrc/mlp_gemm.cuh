@@ -119,7 +119,8 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         // producer
         sm100::tma_prefetch_desc(&tmA);
         sm100::tma_prefetch_desc(&tmB);
-        for (int kb = 0; kb < nk; ++kb) {
+        int kb = 0;
+        for (; kb < nk; ++kb) {
             const int s = kb % STAGES, it = kb / STAGES;
             if (kb >= STAGES && !sm100::mbar_wait(&empty[s], (it - 1) & 1, kWaitLimit)) {
                 *abort_flag = 1;
@@ -132,6 +133,9 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             sm100::tma_load_2d(a, &tmA, &full[s], kb * kGemmBK, m0);
             sm100::tma_load_2d(b, &tmB, &full[s], kb * kGemmBK, n0);
         }
+        // where a role gave up, loads may still be on their way into this block's memory
+        for (int i = kb < STAGES ? 0 : kb - STAGES; i < kb; ++i)
+            sm100::mbar_wait(&full[i % STAGES], (i / STAGES) & 1, kWaitLimit);
     } else if (warp == 1 && lane == 0) {
         // MMA issuer
         constexpr uint32_t idesc = sm100::idesc_bf16_f32(kGemmBM, BN);
