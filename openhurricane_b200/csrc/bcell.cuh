@@ -141,7 +141,7 @@ struct BCell {
         }
         return first;
     }
-    __device__ void keep_matrix(bool) {}   // autoUpdateJacobian takes the cell group
+    static constexpr bool kAuto = false;   // autoUpdateJacobian takes the cell group
 
     // once per block: the places nothing writes later, the term lists
     __device__ void init() {
@@ -354,7 +354,7 @@ struct BCell {
         return __shfl_sync(full, (SL == 2 && p >= 32) ? a[SL - 1][q] : a[0][q], p & 31);
     }
 
-    __device__ __forceinline__ void solve(double (&x)[E]) {
+    __device__ __forceinline__ void solve(double (&x)[E], bool) {
         // the pivot step that row lane + 32 e was chosen in (N and more: not yet, none)
         int at[SL];
 #pragma unroll

@@ -3,9 +3,9 @@
 // a warp, or several warps, integrate together. Every warp of the cell runs
 // it with the same values, so that the control flow is uniform.
 //
-// Cell provides: E elements per lane, has(e) (the lane carries element e),
-// T_of(y), evaluate(y, y0, dt, rhs_only) with f[e] where f_here(),
-// keep_matrix(reuse), solve(x), first_bad(bad) and max_nonneg(v).
+// Cell provides: E elements per lane, kAuto (autoUpdateJacobian is on), has(e) (the lane
+// carries element e), T_of(y), evaluate(y, y0, dt, rhs_only) with f[e] where f_here(),
+// solve(x, reuse) with the last factors where reuse, first_bad(bad) and max_nonneg(v).
 #pragma once
 
 #include "integrator.cuh"
@@ -57,7 +57,7 @@ struct StepControl : Cell {
         int count = 0;
         double lastErr = 0.0, d[E];
         bool on = true, error_pass = false;
-        const bool autoJ = P.auto_update_jacobian != 0;
+        constexpr bool autoJ = Cell::kAuto;
         const int stepJ = P.step_to_update_jac;
         while (true) {
             const bool keepJ = autoJ && !error_pass && count != 0 && count % stepJ != 0;
@@ -70,9 +70,8 @@ struct StepControl : Cell {
                 on = this->f_here();
                 break;
             }
-            if (autoJ) this->keep_matrix(keepJ);
             double x[E];
-            this->solve(x);
+            this->solve(x, keepJ);
             ++n_newton;
             const int bad = this->first_bad(x);
 #pragma unroll

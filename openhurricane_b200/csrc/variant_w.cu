@@ -22,15 +22,15 @@ bool launch_w_fits(const WMech &m, const IntegratorParams &P) {
     return (m.nsp + 1 <= 10 ? w_warps<10>(m, P) : w_warps<16>(m, P)) > 0;
 }
 
-template <int N, int BLOCKS>
+template <int N, int BLOCKS, bool AUTO>
 static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
                     cudaStream_t st, std::string &err) {
-    auto kern = integrate_w_kernel<N, BLOCKS>;
+    auto kern = integrate_w_kernel<N, BLOCKS, AUTO>;
     const int warps = w_warps<N>(m, P);
     const size_t sm = w6_smem_bytes<N>(m, warps, P.auto_update_jacobian != 0);
     int per_sm = 0;
     if (warps > 0) {
-        if (int rc = allow_smem<integrate_w_kernel<N, BLOCKS>>(err)) return rc;
+        if (int rc = allow_smem<integrate_w_kernel<N, BLOCKS, AUTO>>(err)) return rc;
         HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, sm));
     }
     if (per_sm < 1) {
@@ -56,8 +56,10 @@ static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, cons
 template <int N>
 static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
                     cudaStream_t st, std::string &err) {
-    if (io.nqueue < (int64_t)8 * 2 * kWWarps * num_sms) return launch_w<N, 1>(m, num_sms, P, io, st, err);
-    return launch_w<N, 2>(m, num_sms, P, io, st, err);
+    const bool few = io.nqueue < (int64_t)8 * 2 * kWWarps * num_sms;
+    if (P.auto_update_jacobian)
+        return few ? launch_w<N, 1, true>(m, num_sms, P, io, st, err) : launch_w<N, 2, true>(m, num_sms, P, io, st, err);
+    return few ? launch_w<N, 1, false>(m, num_sms, P, io, st, err) : launch_w<N, 2, false>(m, num_sms, P, io, st, err);
 }
 
 int launch_integrate_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,

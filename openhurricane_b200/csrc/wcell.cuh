@@ -41,11 +41,16 @@
 //    2786 Newton iterations instead of 4191 on two of the 4096 Dirichlet cells);
 //  * norms: warp max reductions of the bit patterns.
 //
+// With autoUpdateJacobian the factors stay in shared memory and an iteration that keeps the
+// Jacobian sums f alone and substitutes. That is a build of its own: as an option of one
+// build it made every iteration 6 % longer, and before the factors were kept it saved nothing
+// (1001 Dirichlet cells at 1e-7 s, a Jacobian every ten iterations: 61.7 -> 50.2 ms).
+//
 // Measured (B200, 9 species / 21 reactions): one Newton iteration of the stiffest
-// cell takes 4.8 us (before: 13.9 us with lane i holding row i, the reactions' lists
+// cell takes 4.5 us (before: 13.9 us with lane i holding row i, the reactions' lists
 // walked and the LU's rows broadcast one by one). Flow steps: 4096 Dirichlet cells at
-// 1e-7 s 278 -> 97 ms, 12,288 mixed cells at 1e-5 s 638 -> 351 ms, 1001 cells of the
-// constant-volume reactor 685 -> 91 ms (there against the cell group).
+// 1e-7 s 278 -> 92 ms, 12,288 mixed cells at 1e-5 s 656 -> 347 ms, 1001 cells of the
+// constant-volume reactor 682 -> 88 ms (there against the cell group).
 #pragma once
 
 #include "fastmath.cuh"
@@ -98,6 +103,8 @@ struct WLayout {
     __host__ __device__ static size_t doubles(int nrc, int nrc32, int njob32) {
         return (size_t)kDH + 2 * nrc32 + njob32 + (size_t)LD * (nrc > 0 ? nrc : 1);
     }
+    // autoUpdateJacobian's factors behind it: U, then the multipliers by row (odd strides)
+    static constexpr int kLU = COLS + 1, kLM = N + 1, kFactors = N * (kLU + kLM);
 };
 
 // One reaction in the general form (any orders, up to four participants a
@@ -240,9 +247,11 @@ static __device__ HC_NOINLINE void w_reaction_general(double *s, const double *x
     }
 }
 
-template <int N>
+// AUTO: autoUpdateJacobian; a build of its own, so that the other carries none of it
+template <int N, bool AUTO>
 struct WCell {
     using L = WLayout<N>;
+    static constexpr bool kAuto = AUTO;
     static constexpr int E = 1;       // every lane of a row carries the row's element
     static constexpr unsigned full = 0xffffffffu;
     const WMech &m;
@@ -256,6 +265,8 @@ struct WCell {
     double cvRu;      // Ru in the constant-volume reactor, else 0
     int da, sa, db, sb, dn;   // the dot product this lane evaluates: places, strides, length
     double a[L::C];   // this lane's columns of [I - dt J | rhs]
+    double pinv;      // this row's reciprocal pivot
+    unsigned long long order;   // row of pivot k, 4 bits each
     double f[1];      // this row's right-hand side (where f_here())
 
     __device__ WCell(const WMech &mm, const WTabs6 &t, const IntegratorParams &pp, int at, int l)
@@ -304,18 +315,6 @@ struct WCell {
         const unsigned bad = __ballot_sync(full, act && h == 0 && !finite(x[0]));
         return bad ? __ffs(bad) - 1 : 1 << 30;
     }
-    // autoUpdateJacobian: store the Newton matrix, or take the stored one with the
-    // new right-hand side (it is factored again: the elimination keeps no multipliers)
-    __device__ void keep_matrix(bool reuse) {
-        if (!act) return;
-        double *A = w_smem() + so + L::doubles(m.nrc, m.nrc32, m.njob32) + row * L::COLS + h * L::C;
-#pragma unroll
-        for (int c = 0; c < L::C; ++c) {
-            if (!reuse) A[c] = a[c];
-            else if (h * L::C + c < N) a[c] = A[c];
-        }
-    }
-
     // One reaction's row of D (lanes past the last reaction write nothing); FULL: the
     // round has third-body or fall-off reactions.
     template <bool FULL>
@@ -486,7 +485,23 @@ struct WCell {
         double dot = 0.0;
         const double *Dh = D + (act ? h : 0) * L::C;
         // four entries at a time, so that their table and record loads overlap
-        for (int e = 0; e < m.gE; e += 4) {
+        for (int e = 0; AUTO && rhs_only && e < m.gE; e += 4) {      // column N alone
+            double nu[4], q[4], da_[4], db_[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                nu[k] = *tb.d(tb.gnu + 16 * (e + k) + row);
+                q[k] = D[*tb.i(tb.gslot + 16 * (e + k) + row) * L::LD + N];
+                const int p = (e + k < dn) ? e + k : 0;
+                da_[k] = (e + k < dn) ? s[da + p * sa] : 0.0;
+                db_[k] = s[db + p * sb];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                dot += da_[k] * db_[k];
+                acc[L::cN] += nu[k] * q[k];
+            }
+        }
+        for (int e = 0; !(AUTO && rhs_only) && e < m.gE; e += 4) {
             double nu[4], da_[4], db_[4];
             const double2 *d2[4];
 #pragma unroll
@@ -531,13 +546,41 @@ struct WCell {
         if (h == L::hN) a[L::cN] = (-y + y0[0]) + dt * f[0];
     }
 
-    // x of [A | b] in the registers a[]; every lane gets its row's element
-    __device__ __forceinline__ void solve(double (&x)[1]) {
+    // x of [A | b] in the registers a[]; every lane gets its row's element. reuse (AUTO): with
+    // the factors of the last call and the right-hand side in a[]; step by step what the
+    // elimination does to it, so that x is the same to the last bit
+    __device__ __forceinline__ void solve(double (&x)[1], bool reuse) {
+        double *U = w_smem() + so + L::doubles(m.nrc, m.nrc32, m.njob32), *M = U + N * L::kLU;
+        if (AUTO && reuse) {
+            double b = a[L::cN];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const double u = __shfl_sync(full, b, L::hN * L::R + ((int)(order >> (4 * k)) & 15));
+                b -= M[(act ? row : 0) * L::kLM + k] * u;
+            }
+#pragma unroll
+            for (int c = 0; c < L::C; ++c) a[c] = U[(act ? row : 0) * L::kLU + h * (act ? L::C : 0) + c];
+            substitute(x, b);
+            return;
+        }
+        eliminate(M);
+        if (AUTO) {
+            if (act) {
+#pragma unroll
+                for (int c = 0; c < L::C; ++c) U[row * L::kLU + h * L::C + c] = a[c];
+            }
+            __syncwarp();
+        }
+        substitute(x, a[L::cN]);
+    }
+
+    // M (AUTO): the multipliers
+    __device__ __forceinline__ void eliminate(double *M) {
         // the pivot's key carries its row; a zero pivot makes the reciprocal, and x, not finite
         constexpr int R = L::R;
-        double pinv = 0.0;
+        pinv = 0.0;
         bool used = !act;
-        unsigned long long order = 0ull;      // row of pivot k, 4 bits each
+        order = 0ull;
         auto key = [&](double v, int hk) {
             const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu;
             return (h == hk && !used) ? ((hi & ~31u) | (unsigned)(31 - row)) : 0u;
@@ -555,6 +598,7 @@ struct WCell {
             const int from = h * R + pr;
             used = used || piv;
             const double l = used ? 0.0 : mine * inv;
+            if (AUTO && act && h == 0) M[row * L::kLM + k] = l;
             pinv = piv ? inv : pinv;
             order |= (unsigned long long)pr << (4 * k);
             // the next pivot column first: its search and reciprocals run under the other columns
@@ -571,14 +615,16 @@ struct WCell {
                 a[c] -= l * u;
             }
         }
-        // back substitution along the pivot order, the right-hand side in column block hN
-        double b = a[L::cN];
+    }
+
+    // back substitution along the pivot order; b: the eliminated right-hand side, in column block hN
+    __device__ __forceinline__ void substitute(double (&x)[1], double b) {
         x[0] = 0.0;
 #pragma unroll
         for (int k = N - 1; k >= 0; --k) {
             const int pr = (int)(order >> (4 * k)) & 15;
-            const double u = __shfl_sync(full, a[k % L::C], (k / L::C) * R + rl);
-            const double xk = __shfl_sync(full, b * pinv, L::hN * R + pr);
+            const double u = __shfl_sync(full, a[k % L::C], (k / L::C) * L::R + rl);
+            const double xk = __shfl_sync(full, b * pinv, L::hN * L::R + pr);
             x[0] = (row == k) ? xk : x[0];
             b -= u * xk;
         }
@@ -591,13 +637,13 @@ constexpr int kWWarps = 8;  // most warps (cells in flight) per block
 template <int N>
 size_t w6_smem_bytes(const WMech &m, int warps, bool keepJ) {
     using L = WLayout<N>;
-    const size_t w = L::doubles(m.nrc, m.nrc32, m.njob32) + (keepJ ? (size_t)N * L::COLS : 0);
+    const size_t w = L::doubles(m.nrc, m.nrc32, m.njob32) + (keepJ ? (size_t)L::kFactors : 0);
     return sizeof(double) * (w6_tables_doubles(m) + w * warps);
 }
 
 // BLOCKS an SM: 1 (up to 255 registers a thread, nothing spilled: the shorter Newton
 // iteration) or 2 (128 registers: more cells in flight); variant_w.cu chooses
-template <int N, int BLOCKS>
+template <int N, int BLOCKS, bool AUTO>
 __global__ void __launch_bounds__(32 * kWWarps, BLOCKS)
 integrate_w_kernel(const __grid_constant__ WMech m, const __grid_constant__ IntegratorParams P,
                    const __grid_constant__ CellIO io) {
@@ -629,7 +675,7 @@ integrate_w_kernel(const __grid_constant__ WMech m, const __grid_constant__ Inte
         tb.rx = copyi(m.rx, 2 * m.nrc32);
         tb.gslot = copyi(m.gslot, 16 * m.gE);
     }
-    const size_t wd = L::doubles(m.nrc, m.nrc32, m.njob32) + (P.auto_update_jacobian ? (size_t)N * L::COLS : 0);
+    const size_t wd = L::doubles(m.nrc, m.nrc32, m.njob32) + (AUTO ? (size_t)L::kFactors : 0);
     const int so = (int)(w6_tables_doubles(m) + (size_t)warp * wd);
     double *s = w_smem() + so;
     for (int i = lane; i < (int)wd; i += 32) s[i] = 0.0;
@@ -641,7 +687,7 @@ integrate_w_kernel(const __grid_constant__ WMech m, const __grid_constant__ Inte
         s[L::kA3 + 2 * kWOne] = 1.0;
     }
     __syncthreads();
-    StepControl<WCell<N>> ci(m, tb, P, so, lane);
+    StepControl<WCell<N, AUTO>> ci(m, tb, P, so, lane);
     const int row = ci.row;
     const bool sp = ci.act && row < nsp, own = sp && ci.h == 0;
     const double W = sp ? *tb.d(kWW * 32 + row) : 1.0;
