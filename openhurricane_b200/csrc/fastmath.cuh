@@ -67,7 +67,7 @@ __device__ __forceinline__ double lean_exp(double x) {
 }
 
 // 1/b for positive normal b: the hardware approximation and one cubic step
-// r (1 + e + e^2), e = 1 - b r, which triples its correct bits
+// r (1 + e + e^2), e = 1 - b r, which triples its correct bits (frcp, rtc_base.cuh)
 __device__ __forceinline__ double fast_rcp(double b) {
 #ifdef __CUDA_ARCH__
     double r;
@@ -83,6 +83,8 @@ __device__ __forceinline__ double fast_rcp(double b) {
 // ln(1 + f) = f - (f^2/2 - s (f^2/2 + R)), R = 2/3 s^2 + 2/5 s^4 + ... (the series of
 // 2 artanh s; ten terms, truncation 1e-18), in two chains like fast_exp and without a
 // branch (the library's log takes 294 cycles on a B200). Within 1 ulp of the exact value.
+// The reduction, ln 2 in two parts and the order of the last sum are those of fdlibm's log
+// (K. C. Ng, SunSoft 1993); its fitted coefficients are not used.
 __device__ __forceinline__ double fast_log(double x) {
     const bool low = x < 2.2250738585072014e-308;          // below the normal range (or not positive)
     const double xs = low ? x * 18014398509481984.0 : x;   // 2^54

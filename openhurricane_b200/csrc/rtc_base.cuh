@@ -59,8 +59,10 @@ __device__ __forceinline__ double pow_n(double x, double y) {
 
 // 1/b without a branch to a slow path: the hardware approximation r (PTX
 // rcp.approx.ftz.f64, 2^-20) and one cubic step r (1 + e + e^2), e = 1 - b r,
-// which triples its correct bits in three dependent operations; the result is
-// within an ulp of the correctly rounded reciprocal. Zero, infinity and NaN
+// which triples its correct bits in three dependent operations (the third-order
+// member of Schroeder's iterations, 1870, on the multiply-add residual of
+// Markstein, IBM J. Res. Dev. 34 (1990) 111-119); the result is within an ulp of
+// the correctly rounded reciprocal. Zero, infinity and NaN
 // keep the approximation's own result (+-inf, +-0, NaN), as do subnormal b
 // (flushed: +-inf).
 __device__ __forceinline__ double frcp(double b) {

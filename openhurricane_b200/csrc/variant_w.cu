@@ -52,11 +52,16 @@ static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, cons
 // larger number in flight pay. Dirichlet cells at 1e-7 s and mixed cells at 1e-6 s, ms,
 // first / second build: 12,288 cells 118 / 162 and 79 / 97; 18,944: 182 / 182 and
 // 118 / 108; 37,888: 361 / 318 and 239 / 234; 131,072 mixed: 779 / 674. So the line lies
-// at 8 cells for each of the second's warps.
+// at 8 cells for each of the second's warps. Where shared memory holds one block only
+// (mechanisms with many reactions) the second build would be the first with spills:
+// 15 species / 45 reactions, first / second: 20,000 cells 266 / 320 ms, 40,000 486 / 577.
 template <int N>
 static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,
                     cudaStream_t st, std::string &err) {
-    const bool few = io.nqueue < (int64_t)8 * 2 * kWWarps * num_sms;
+    const int warps = w_warps<N>(m, P);
+    const size_t sm = w6_smem_bytes<N>(m, warps, P.auto_update_jacobian != 0);
+    const bool two = 2 * (sm + 1024) <= 228 * 1024;       // blocks an SM by shared memory
+    const bool few = !two || io.nqueue < (int64_t)8 * 2 * warps * num_sms;
     if (P.auto_update_jacobian)
         return few ? launch_w<N, 1, true>(m, num_sms, P, io, st, err) : launch_w<N, 2, true>(m, num_sms, P, io, st, err);
     return few ? launch_w<N, 1, false>(m, num_sms, P, io, st, err) : launch_w<N, 2, false>(m, num_sms, P, io, st, err);

@@ -221,3 +221,29 @@ def test_a_kept_jacobian_shortens_the_iteration(tmp_path):
         per[auto] = best
     assert per[1] <= 0.9 * per[0], per
     m.close()
+
+
+def test_more_cells_do_not_take_a_build_that_does_not_fit_twice(tmp_path):
+    """The build for two blocks an SM pays where shared memory holds two. With 15 species and
+    45 reactions it holds one: a ninth more cells (18,000 and 20,000 lie on both sides of
+    the line for 148 SMs) may take a fifth more time. (The other build took a third more.)"""
+    from openhurricane_b200.chemistry import ChemistrySource, Flow, Mechanism
+    dev = _dev()
+    d = lambda a: torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device=dev)
+    t = slower(_tables(15, 45, 8, 3, tmp_path))
+    c, rho = _states(t, 200)
+    m, took = Mechanism(t), {}
+    for n in (90, 100):
+        state = [np.tile(a, n) for a in (c.T, c.p, rho, c.Y)]
+        took[n] = np.inf
+        for _ in range(2):
+            cs = ChemistrySource(m, Flow(*[d(a) for a in state]), **OPTS)
+            dt = torch.full((200 * n,), 1e-8, dtype=torch.float64, device=dev)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            cs.solveUpdate(dt, 1.0)
+            b.record()
+            torch.cuda.synchronize()
+            took[n] = min(took[n], a.elapsed_time(b))
+    assert took[100] <= 1.2 * took[90], took
+    m.close()
