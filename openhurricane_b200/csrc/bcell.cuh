@@ -29,8 +29,8 @@
 // Measured (B200, 53 species / 325 reactions): one Newton iteration of one cell takes
 // 20.5 us with two cells on an SM (before: 143 us in the cell group of 64 lanes; with
 // four warps a cell 28.5 us), a pivot step 450 cycles and a step of the substitution
-// about 60; 768 cells, flow step of 1e-7 s: 948 -> 239 ms; 8191 Jacobians and
-// right-hand sides: 1482 -> 282 us.
+// about 60; 768 cells, flow step of 1e-7 s: 945 -> 244 ms; 8191 Jacobians and
+// right-hand sides: 1487 -> 283 us.
 #pragma once
 
 #include "rates.cuh"

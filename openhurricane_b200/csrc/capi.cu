@@ -1225,9 +1225,10 @@ static int integrate_impl(hc_mech_t m, const hc_opts *opts, int64_t ncells, doub
                         "SRI, explicit reverse (REV), PLOG, HIGH, LT, JAN, FIT1 or collision rate laws");
         return launch_integrate_s(m->w, m->num_sms, P, io, st, g_err);
     }
-    // automatic choice (kernel 0): the warp-per-cell kernel wherever it takes
-    // the mechanism (the fastest on the batched workload: 1.14e8 Newton
-    // iterations/s against 0.6e8 for the cell group), else the cell group
+    // automatic choice (kernel 0): the warp-per-cell kernel wherever it takes the
+    // mechanism (2.2e8 Newton iterations/s on the batched workload, the cell group
+    // 0.6e8), the block-per-cell kernel above 16 unknowns (20.5 us an iteration of 54
+    // unknowns, the cell group 143), else the cell group
     const bool auto_w = m->kernel == 0 && m->w_ok && launch_w_fits(m->w, P);
     if (m->kernel == 6 || auto_w) {
         if (!auto_w && (!m->w_ok || opts->reactor != 0))

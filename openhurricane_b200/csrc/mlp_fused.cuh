@@ -18,8 +18,9 @@
 // Shapes: up to kFusedLayers layers, inputs and widths up to 256, outputs up to
 // 256; anything else takes the layer-by-layer form.
 //
-// Measured (B200, an ensemble's predictions, 12-256-256-256-10, fused / layer by
-// layer): 4,096 rows 146 / 205 us, 65,536 rows 268 / 548 us, 300,000 rows 985 / 2497 us.
+// Measured (B200, an ensemble's forward passes, three networks 12-256-256-256-10, fused /
+// layer by layer with an earlier form of GELU): 4,096 rows 123 / 205 us, 65,536 rows
+// 233 / 548 us, 300,000 rows 866 / 2497 us.
 #pragma once
 
 #include "mlp_gemm.cuh"

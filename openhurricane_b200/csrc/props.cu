@@ -30,7 +30,7 @@
 // registers) and gain nothing over the former kernel, which had one chain too.
 //
 // Measured (B200, 65,536 cells of 53 species): 1911 us before (a warp per cell, a
-// division and a square root a pair), 270 us now.
+// division and a square root a pair), 280 us now.
 #include <cuda_runtime.h>
 
 #include <string>

@@ -9,8 +9,8 @@
 // and one 32-byte load from shared memory, a lane sums its reactions' contributions
 // in its own column of shared memory and the columns are added last. Measured
 // (B200) against a 32- or 64-lane group per cell with list walks: 1,048,576 cells of
-// 9 species 3779 -> 219 us, 65,536 of 53 species 3467 -> 399 us, implicit terms
-// of 262,144 cells of 9 species (which formed the whole Jacobian) 3290 -> 152 us.
+// 9 species 3777 -> 219 us, 65,536 of 53 species 3471 -> 397 us, implicit terms
+// of 262,144 cells of 9 species (which formed the whole Jacobian) 3292 -> 152 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>

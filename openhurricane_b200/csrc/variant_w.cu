@@ -48,12 +48,12 @@ static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, cons
 
 // One block of eight warps per SM and no spills, or two with 128 registers a thread.
 // A flow step ends with its stiffest cells, whose iterations the first build does in
-// 4.8 us against 6.5 us; only when the cells go round many times does the second's
-// larger number in flight pay. Dirichlet cells at 1e-7 s and mixed cells at 1e-6 s, ms,
-// first / second build: 12,288 cells 118 / 162 and 79 / 97; 18,944: 182 / 182 and
-// 118 / 108; 37,888: 361 / 318 and 239 / 234; 131,072 mixed: 779 / 674. So the line lies
-// at 8 cells for each of the second's warps. Where shared memory holds one block only
-// (mechanisms with many reactions) the second build would be the first with spills:
+// 4.5 us against 6.5 us; only when the cells go round many times does the second's
+// larger number in flight pay. First / second build in ms, Dirichlet cells at 1e-7 s, mixed
+// cells at 1e-6 s and at 1e-5 s: 12,288 cells 116 / 158, 79 / 100 and 320 / 421; 18,944
+// 175 / 180, 121 / 114 and 493 / 513; 37,888 348 / 309, 243 / 211 and 980 / 859. So the
+// line lies at 8 cells for each of the second's warps. Where shared memory holds one block
+// only (mechanisms with many reactions) the second build would be the first with spills:
 // 15 species / 45 reactions, first / second: 20,000 cells 266 / 320 ms, 40,000 486 / 577.
 template <int N>
 static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, const CellIO &io,

@@ -51,8 +51,8 @@
 // Measured (B200, 9 species / 21 reactions): one Newton iteration of the stiffest
 // cell takes 4.5 us (before: 13.9 us with lane i holding row i, the reactions' lists
 // walked and the LU's rows broadcast one by one). Flow steps: 4096 Dirichlet cells at
-// 1e-7 s 278 -> 92 ms, 12,288 mixed cells at 1e-5 s 656 -> 347 ms, 1001 cells of the
-// constant-volume reactor 682 -> 88 ms (there against the cell group).
+// 1e-7 s 277 -> 92 ms, 12,288 mixed cells at 1e-5 s 641 -> 335 ms, 1001 cells of the
+// constant-volume reactor 684 -> 86 ms (there against the cell group).
 #pragma once
 
 #include "fastmath.cuh"
