@@ -26,12 +26,10 @@ constexpr size_t kMaxSmem = 227 * 1024;   // shared memory a block can have
 // kernel, not to the launch, so every caller names the same number: kMaxSmem where the
 // size of a launch depends on the mechanism or the cells (a thread with a small launch
 // would otherwise lower it between another thread's call and launch). Called for each
-// launch, 0.06 to 0.3 us (B200, a launch 2.6 us): the limit also belongs to the context, so
-// a remembered "done" would outlive it. A launch that needs no more than every kernel may
-// have goes without (the small calls of a few microseconds).
+// launch, 0.06 us (B200, a launch 2.6 us): the limit also belongs to the context, so a
+// remembered "done" would outlive it.
 template <auto Kernel>
-int allow_smem(size_t need, std::string &err, size_t bytes = kMaxSmem) {
-    if (need <= 48 * 1024) return HC_OK;
+int allow_smem(std::string &err, size_t bytes = kMaxSmem) {
     HC_LCUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     return HC_OK;
 }

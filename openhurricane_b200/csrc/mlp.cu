@@ -92,7 +92,7 @@ int launch_bn(const CUtensorMap &ta, const CUtensorMap &tb, int M, int N, int K,
     auto kern = gemm_bf16_tn_kernel<BN, STAGES>;
     const size_t smem = (size_t)STAGES * GemmSmem<BN>::kStage + 1024 + 256;
     std::string msg;
-    if (int rc = allow_smem<gemm_bf16_tn_kernel<BN, STAGES>>(smem, msg, smem)) return mfail(rc, msg);
+    if (int rc = allow_smem<gemm_bf16_tn_kernel<BN, STAGES>>(msg, smem)) return mfail(rc, msg);
     dim3 grid(M / kGemmBM, N / BN);
     kern<<<grid, 128, smem, st>>>(ta, tb, K, ep, err);
     MCUDA(cudaGetLastError());
@@ -358,7 +358,7 @@ int forward_fused(hc_mlp_t m, const float *X, int64_t B, float *Y, cudaStream_t 
     MCUDA(cudaGetDevice(&dev));
     MCUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     std::string err;
-    if (int rc = allow_smem<mlp_fused_kernel>(FusedSmem::bytes(), err, FusedSmem::bytes())) return mfail(rc, err);
+    if (int rc = allow_smem<mlp_fused_kernel>(err, FusedSmem::bytes())) return mfail(rc, err);
     const int64_t pairs = (B + 2 * kGemmBM - 1) / (2 * kGemmBM);
     const int grid = (int)(pairs < sms ? pairs : sms);
     mlp_fused_kernel<<<grid, kFusedThreads, FusedSmem::bytes(), st>>>(f, X, B, Y, m->err);

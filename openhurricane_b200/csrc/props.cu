@@ -230,7 +230,7 @@ int launch_properties(const DevMech &m, int64_t n, const double *T, const double
     auto smem = [&](int b) { return sizeof(double) * (12 * (size_t)NB * m.nsp + 4 * NB + kPropSp * m.nsp + (2 * m.nsp + 3 * L) * (size_t)b); };
     while (B > 32 && (smem(B) > kMaxSmem || (n + B - 1) / B < sms)) B /= 2;
     const size_t sm = smem(B);
-    if (int rc = allow_smem<properties_kernel>(sm, err)) return rc;
+    if (int rc = allow_smem<properties_kernel>(err)) return rc;
     int per_sm = 0;
     HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, properties_kernel, B * L, sm));
     if (per_sm < 1) {

@@ -208,11 +208,11 @@ template <int L>
 static int launch_lanes(const RMech &m, const DevMech &dm, int64_t n, const double *T, const double *rho,
                         const double *Y, double *Ri, double *diag, cudaStream_t st, std::string &err) {
     const bool imp = diag != nullptr;
+    const int rc = imp ? allow_smem<rates_kernel<true, L>>(err) : allow_smem<rates_kernel<false, L>>(err);
+    if (rc != HC_OK) return rc;
     constexpr int B = kThreads / L;
     const unsigned grid = (unsigned)((n + B - 1) / B);
     const size_t sm = rates_smem(m.nsp, m.nrc, L, imp);
-    const int rc = imp ? allow_smem<rates_kernel<true, L>>(sm, err) : allow_smem<rates_kernel<false, L>>(sm, err);
-    if (rc != HC_OK) return rc;
     if (imp) rates_kernel<true, L><<<grid, kThreads, sm, st>>>(m, dm, n, T, rho, Y, Ri, diag);
     else rates_kernel<false, L><<<grid, kThreads, sm, st>>>(m, dm, n, T, rho, Y, Ri, nullptr);
     HC_LCUDA(cudaGetLastError());

@@ -27,7 +27,7 @@ bool launch_b_fits(const RMech &m, const BMech &b) {
 template <auto Kernel>
 static int b_grid(size_t sm, int num_sms, int64_t n, int64_t &grid, std::string &err) {
     int per_sm = 0;
-    if (int rc = allow_smem<Kernel>(sm, err)) return rc;
+    if (int rc = allow_smem<Kernel>(err)) return rc;
     HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, Kernel, kBThreads, sm));
     if (per_sm < 1) {
         err = "block-per-cell kernel does not fit on an SM";

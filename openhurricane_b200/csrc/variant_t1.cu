@@ -17,7 +17,7 @@ static int launch_t1(const DevMech &m, int num_sms, const IntegratorParams &P, c
     using L = T1Layout<N>;
     auto kern = integrate_t1_kernel<N>;
     const size_t sm = (sizeof(double) * L::kSlots + sizeof(int) * L::kPivSlots) * (size_t)block;
-    if (int rc = allow_smem<integrate_t1_kernel<N>>(sm, err)) return rc;
+    if (int rc = allow_smem<integrate_t1_kernel<N>>(err)) return rc;
     int per_sm = 0;
     HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, sm));
     if (per_sm < 1) {

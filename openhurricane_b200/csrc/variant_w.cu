@@ -30,7 +30,7 @@ static int launch_w(const WMech &m, int num_sms, const IntegratorParams &P, cons
     const size_t sm = w6_smem_bytes<N>(m, warps, P.auto_update_jacobian != 0);
     int per_sm = 0;
     if (warps > 0) {
-        if (int rc = allow_smem<integrate_w_kernel<N, BLOCKS, AUTO>>(sm, err)) return rc;
+        if (int rc = allow_smem<integrate_w_kernel<N, BLOCKS, AUTO>>(err)) return rc;
         HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, sm));
     }
     if (per_sm < 1) {
@@ -85,7 +85,7 @@ static int launch_s(const WMech &m, int num_sms, const IntegratorParams &P, cons
                       sizeof(double) * SLayout<N>::doubles(m.nrc, m.njob) * G * kSWarps;
     int per_sm = 0;
     if (sm <= kMaxSmem) {
-        if (int rc = allow_smem<integrate_s_kernel<N>>(sm, err)) return rc;
+        if (int rc = allow_smem<integrate_s_kernel<N>>(err)) return rc;
             HC_LCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kSWarps, sm));
     }
     if (per_sm < 1) {
