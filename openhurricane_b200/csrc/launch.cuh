@@ -26,8 +26,8 @@ constexpr size_t kMaxSmem = 227 * 1024;   // shared memory a block can have
 // kernel, not to the launch, so every caller names the same number: kMaxSmem where the
 // size of a launch depends on the mechanism or the cells (a thread with a small launch
 // would otherwise lower it between another thread's call and launch). Called for each
-// launch, 0.06 us (B200, a launch 2.6 us): the limit also belongs to the context, so a
-// remembered "done" would outlive it.
+// launch, 0.06 to 0.3 us (B200, a launch 2.6 us): the limit also belongs to the context, so
+// a remembered "done" would outlive it.
 template <auto Kernel>
 int allow_smem(std::string &err, size_t bytes = kMaxSmem) {
     HC_LCUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));

@@ -205,14 +205,18 @@ static int choose_lanes(int nsp, int nrc, int64_t n, int num_sms, bool imp) {
 }
 
 template <int L>
-static int launch_lanes(const RMech &m, const DevMech &dm, int64_t n, const double *T, const double *rho,
+static int launch_lanes(const RMech &m, const DevMech &dm, int num_sms, int64_t n, const double *T, const double *rho,
                         const double *Y, double *Ri, double *diag, cudaStream_t st, std::string &err) {
     const bool imp = diag != nullptr;
-    const int rc = imp ? allow_smem<rates_kernel<true, L>>(err) : allow_smem<rates_kernel<false, L>>(err);
-    if (rc != HC_OK) return rc;
     constexpr int B = kThreads / L;
     const unsigned grid = (unsigned)((n + B - 1) / B);
     const size_t sm = rates_smem(m.nsp, m.nrc, L, imp);
+    // a block alone on its SM and within the default limit goes without: 257 cells of 9
+    // species, a call bound by its host side, 8.4 -> 8.1 us (it varies by 3 %)
+    if (sm > 48 * 1024 || grid > (unsigned)num_sms) {
+        const int rc = imp ? allow_smem<rates_kernel<true, L>>(err) : allow_smem<rates_kernel<false, L>>(err);
+        if (rc != HC_OK) return rc;
+    }
     if (imp) rates_kernel<true, L><<<grid, kThreads, sm, st>>>(m, dm, n, T, rho, Y, Ri, diag);
     else rates_kernel<false, L><<<grid, kThreads, sm, st>>>(m, dm, n, T, rho, Y, Ri, nullptr);
     HC_LCUDA(cudaGetLastError());
@@ -222,12 +226,12 @@ static int launch_lanes(const RMech &m, const DevMech &dm, int64_t n, const doub
 int launch_rates(const RMech &m, const DevMech &dm, int num_sms, int64_t n, const double *T, const double *rho,
                  const double *Y, double *Ri, double *diag, cudaStream_t st, std::string &err) {
     switch (choose_lanes(m.nsp, m.nrc, n, num_sms, diag != nullptr)) {
-    case 1: return launch_lanes<1>(m, dm, n, T, rho, Y, Ri, diag, st, err);
-    case 2: return launch_lanes<2>(m, dm, n, T, rho, Y, Ri, diag, st, err);
-    case 4: return launch_lanes<4>(m, dm, n, T, rho, Y, Ri, diag, st, err);
-    case 8: return launch_lanes<8>(m, dm, n, T, rho, Y, Ri, diag, st, err);
-    case 16: return launch_lanes<16>(m, dm, n, T, rho, Y, Ri, diag, st, err);
-    default: return launch_lanes<32>(m, dm, n, T, rho, Y, Ri, diag, st, err);
+    case 1: return launch_lanes<1>(m, dm, num_sms, n, T, rho, Y, Ri, diag, st, err);
+    case 2: return launch_lanes<2>(m, dm, num_sms, n, T, rho, Y, Ri, diag, st, err);
+    case 4: return launch_lanes<4>(m, dm, num_sms, n, T, rho, Y, Ri, diag, st, err);
+    case 8: return launch_lanes<8>(m, dm, num_sms, n, T, rho, Y, Ri, diag, st, err);
+    case 16: return launch_lanes<16>(m, dm, num_sms, n, T, rho, Y, Ri, diag, st, err);
+    default: return launch_lanes<32>(m, dm, num_sms, n, T, rho, Y, Ri, diag, st, err);
     }
 }
 
